@@ -50,52 +50,60 @@ __device__ __forceinline__ float d2(float v, float k, float a, float b, float c)
   return v * v * k * (a + b - 2.0f * c);
 }
 
-// Two-way value of one cell before the absorbing blend, any region: frame
-// (processBoundary part (i), fd.cpp:1057-1091), 2nd order rings 1-3
-// (modeling2D_low, :1226-1241) or 8th order (modeling2D_high, :1259-1270).
-template <class A>
-__device__ float twoway_cell(const A &cur, const A &prev, const A &V, const ShotDev &g, int ix,
-                             int iz) {
+// Two-way value of one frame cell (edge row or column of the grid) before the
+// absorbing blend (processBoundary part (i), fd.cpp:1057-1091).
+template <class A, class AP, class AV>
+__device__ __forceinline__ float frame_cell(const A &cur, const AP &prev, const AV &V,
+                                            const ShotDev &g, int ix, int iz) {
   const int NX = g.NX, NZ = g.NZ;
-  float c = cur(ix, iz);
-  float p = prev(ix, iz);
-  bool fx = (ix == 0 || ix == NX - 1), fz = (iz == 0 || iz == NZ - 1);
-  if (fx || fz) {
-    float u;
-    if (fx && fz) {
-      u = 2.0f * c - p;
-    } else if (fz) {  // top / bottom rows, fd.cpp:1060-1063
-      u = d2(V(ix, iz), g.kx, cur(ix + 1, iz), cur(ix - 1, iz), c) + 2.0f * c - p;
-    } else if (ix == 0) {  // left column, fd.cpp:1065
-      u = d2(V(ix, iz), g.kz, cur(ix, iz + 1), cur(ix, iz - 1), c) + 2.0f * c - p;
-    } else {  // right column uses the x coefficient, fd.cpp:1066
-      u = d2(V(ix, iz), g.kx, cur(ix, iz + 1), cur(ix, iz - 1), c) + 2.0f * c - p;
-    }
-    if (fz) {  // normal extrapolation along z, fd.cpp:1072-1081
-      int s1 = iz == 0 ? 1 : NZ - 2, s2 = iz == 0 ? 2 : NZ - 3, dz = iz == 0 ? 1 : -1;
-      float y1 = d2(V(ix, s1), g.kz, cur(ix, s1 + dz), cur(ix, s1 - dz), cur(ix, s1));
-      float y2 = d2(V(ix, s2), g.kz, cur(ix, s2 + dz), cur(ix, s2 - dz), cur(ix, s2));
-      u = u + (y1 * 2.0f - y2);
-    }
-    if (fx) {  // normal extrapolation along x, fd.cpp:1082-1091
-      int s1 = ix == 0 ? 1 : NX - 2, s2 = ix == 0 ? 2 : NX - 3, dx = ix == 0 ? 1 : -1;
-      float y1 = d2(V(s1, iz), g.kx, cur(s1 + dx, iz), cur(s1 - dx, iz), cur(s1, iz));
-      float y2 = d2(V(s2, iz), g.kx, cur(s2 + dx, iz), cur(s2 - dx, iz), cur(s2, iz));
-      u = u + (y1 * 2.0f - y2);
-    }
-    return u;
+  const float c = cur(ix, iz);
+  const float p = prev(ix, iz);
+  const bool fx = (ix == 0 || ix == NX - 1), fz = (iz == 0 || iz == NZ - 1);
+  float u;
+  if (fx && fz) {
+    u = 2.0f * c - p;
+  } else if (fz) {  // top / bottom rows, fd.cpp:1060-1063
+    u = d2(V(ix, iz), g.kx, cur(ix + 1, iz), cur(ix - 1, iz), c) + 2.0f * c - p;
+  } else {  // left column, fd.cpp:1065; the right one uses the x coefficient, :1066
+    u = d2(V(ix, iz), ix == 0 ? g.kz : g.kx, cur(ix, iz + 1), cur(ix, iz - 1), c) + 2.0f * c - p;
   }
-  Coef k = coef(V(ix, iz), g);
-  float uzz, uxx;
-  if (ix >= 4 && ix <= NX - 5 && iz >= 4 && iz <= NZ - 5) {
-    uzz = lap8(cur(ix, iz - 4), cur(ix, iz - 3), cur(ix, iz - 2), cur(ix, iz - 1), c,
-               cur(ix, iz + 1), cur(ix, iz + 2), cur(ix, iz + 3), cur(ix, iz + 4));
-    uxx = lap8(cur(ix - 4, iz), cur(ix - 3, iz), cur(ix - 2, iz), cur(ix - 1, iz), c,
-               cur(ix + 1, iz), cur(ix + 2, iz), cur(ix + 3, iz), cur(ix + 4, iz));
-  } else {
-    uzz = cur(ix, iz - 1) + cur(ix, iz + 1) - 2.0f * c;
-    uxx = cur(ix + 1, iz) + cur(ix - 1, iz) - 2.0f * c;
+  if (fz) {  // normal extrapolation along z, fd.cpp:1072-1081
+    const int dz = iz == 0 ? 1 : -1, s1 = iz + dz, s2 = s1 + dz;
+    const float y1 = d2(V(ix, s1), g.kz, cur(ix, s1 + dz), cur(ix, s1 - dz), cur(ix, s1));
+    const float y2 = d2(V(ix, s2), g.kz, cur(ix, s2 + dz), cur(ix, s2 - dz), cur(ix, s2));
+    u = u + (y1 * 2.0f - y2);
   }
+  if (fx) {  // normal extrapolation along x, fd.cpp:1082-1091
+    const int dx = ix == 0 ? 1 : -1, s1 = ix + dx, s2 = s1 + dx;
+    const float y1 = d2(V(s1, iz), g.kx, cur(s1 + dx, iz), cur(s1 - dx, iz), cur(s1, iz));
+    const float y2 = d2(V(s2, iz), g.kx, cur(s2 + dx, iz), cur(s2 - dx, iz), cur(s2, iz));
+    u = u + (y1 * 2.0f - y2);
+  }
+  return u;
+}
+
+// Two-way value of a cell in the 2nd-order rings 1-3 (modeling2D_low,
+// :1226-1241), its velocity v given.
+template <class A, class AP>
+__device__ __forceinline__ float twoway_low(const A &cur, const AP &prev, float v,
+                                            const ShotDev &g, int ix, int iz) {
+  const float c = cur(ix, iz), p = prev(ix, iz);
+  const Coef k = coef(v, g);
+  const float uzz = cur(ix, iz - 1) + cur(ix, iz + 1) - 2.0f * c;
+  const float uxx = cur(ix + 1, iz) + cur(ix - 1, iz) - 2.0f * c;
+  return k.vz * uzz + k.vx * uxx + 2.0f * c - p;
+}
+
+// The same of a cell in the 8th-order region (modeling2D_high, :1259-1270).
+template <class A, class AP>
+__device__ __forceinline__ float twoway_high(const A &cur, const AP &prev, float v,
+                                             const ShotDev &g, int ix, int iz) {
+  const float c = cur(ix, iz), p = prev(ix, iz);
+  const Coef k = coef(v, g);
+  const float uzz = lap8(cur(ix, iz - 4), cur(ix, iz - 3), cur(ix, iz - 2), cur(ix, iz - 1), c,
+                         cur(ix, iz + 1), cur(ix, iz + 2), cur(ix, iz + 3), cur(ix, iz + 4));
+  const float uxx = lap8(cur(ix - 4, iz), cur(ix - 3, iz), cur(ix - 2, iz), cur(ix - 1, iz), c,
+                         cur(ix + 1, iz), cur(ix + 2, iz), cur(ix + 3, iz), cur(ix + 4, iz));
   return k.vz * uzz + k.vx * uxx + 2.0f * c - p;
 }
 
@@ -197,9 +205,9 @@ __device__ __forceinline__ Absorb absorb_geom(const A &V, const ShotDev &g, int 
 
 // Absorbing blend of one field at one cell with two-way value u3.  U3 =
 // two-way field (tile + 1 halo); cur/P = current and previous field.
-template <class U3A, class A>
+template <class U3A, class A, class AP>
 __device__ __forceinline__ float absorb_apply(const Absorb &q, float u3, const U3A &U3,
-                                              const A &cur, const A &P, const ShotDev &g, int ix,
+                                              const A &cur, const AP &P, const ShotDev &g, int ix,
                                               int iz) {
   if (q.kind == 0) return u3 + 0.0f;
   float u31;

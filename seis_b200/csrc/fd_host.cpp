@@ -154,7 +154,7 @@ struct Plan {
   float *d_taps = nullptr;
   float *d_stage = nullptr;  // staging for unpadded uploads / transposes
   size_t stage_elems = 0;
-  int NT = 0, nt = 0, ndel = 0, max_strip = 0, max_NZ = 0;
+  int NT = 0, nt = 0, ndel = 0, max_strip = 0, max_NZ = 0, max_tab = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   int64_t launches_per_run = 0;
@@ -347,13 +347,15 @@ int encode_maps(Plan &p, std::vector<ShotDev> &sds, CUtensorMap **d_out) {
     int rc = SEIS_OK;
     for (int k = 0; k < 3 && !rc; k++) {
       rc = encode_map(p.ctx, g, g.fa[k], rows, wide, &m[MAP_FA_WIDE + k]);
-      if (!rc) rc = encode_map(p.ctx, g, g.fa[k], rows, narrow, &m[MAP_FA_NARROW + k]);
+      if (!rc) rc = encode_map(p.ctx, g, g.fa[k], rows - 8, narrow, &m[MAP_FA_PREV + k]);
+      if (!rc && p.op == OP_BORN_ADJ)
+        rc = encode_map(p.ctx, g, g.fa[k], rows, narrow, &m[MAP_FA_NARROW + k]);
       if (!rc && g.fb[k]) rc = encode_map(p.ctx, g, g.fb[k], rows, wide, &m[MAP_FB_WIDE + k]);
-      if (!rc && g.fb[k]) rc = encode_map(p.ctx, g, g.fb[k], rows, narrow, &m[MAP_FB_NARROW + k]);
+      if (!rc && g.fb[k]) rc = encode_map(p.ctx, g, g.fb[k], rows - 8, narrow, &m[MAP_FB_PREV + k]);
     }
-    if (!rc) rc = encode_map(p.ctx, g, g.vel, rows, narrow, &m[MAP_VEL]);
-    if (!rc) rc = encode_map(p.ctx, g, g.vel, rows, wide, &m[MAP_VEL_WIDE]);
-    if (!rc && g.dv) rc = encode_map(p.ctx, g, g.dv, rows, narrow, &m[MAP_DV]);
+    if (!rc) rc = encode_map(p.ctx, g, g.vel, rows - 8, narrow, &m[MAP_VEL_PREV]);
+    if (!rc && p.op == OP_BORN_ADJ)
+      rc = encode_map(p.ctx, g, g.vel, rows, wide, &m[MAP_VEL_WIDE]);
     // interior tiles
     const int TX = shape_tx(p.shape), TZ = shape_tz(p.shape);
     for (int k = 0; k < 3 && !rc; k++) {
@@ -363,7 +365,8 @@ int encode_maps(Plan &p, std::vector<ShotDev> &sds, CUtensorMap **d_out) {
       if (!rc && g.fb[k]) rc = encode_map(p.ctx, g, g.fb[k], TZ, TX, &m[MAP_FB_TILE + k]);
     }
     if (!rc) rc = encode_map(p.ctx, g, g.vel, TZ, TX, &m[MAP_VEL_TILE]);
-    if (!rc) rc = encode_map(p.ctx, g, g.vel, TZ + 2 * HI, TX + 2 * HI, &m[MAP_VEL_HALO]);
+    if (!rc && p.op == OP_BORN_ADJ)
+      rc = encode_map(p.ctx, g, g.vel, TZ + 2 * HI, TX + 2 * HI, &m[MAP_VEL_HALO]);
     if (!rc && g.dv) rc = encode_map(p.ctx, g, g.dv, TZ, TX, &m[MAP_DV_TILE]);
     if (rc) return rc;
   }
@@ -447,7 +450,7 @@ int plan_create(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *descs
     if (op == OP_BORN || op == OP_RTM || op == OP_BORN_PLANE || op == OP_RTM_PLANE ||
         op == OP_RTM_TRUE || op == OP_RTM_UPDOWN)
       for (int k = 0; k < 3 && rc == SEIS_OK; k++) rc = alloc_field(*p, g, &g.fb[k]);
-    float *vel = nullptr, *dv = nullptr, *wav = nullptr, *rec = nullptr;
+    float *vel = nullptr, *dv = nullptr, *wav = nullptr, *rec = nullptr, *ptab = nullptr;
     int *gzd = nullptr;
     if (rc == SEIS_OK) rc = alloc_field(*p, g, &vel);
     if (rc == SEIS_OK && (op == OP_BORN || op == OP_BORN_PLANE)) rc = alloc_field(*p, g, &dv);
@@ -459,6 +462,8 @@ int plan_create(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *descs
     if (rc == SEIS_OK) rc = p->alloc(&wav, (size_t)g.NT);
     if (rc == SEIS_OK) rc = p->alloc(&rec, (size_t)d.nt * d.nx);
     if (rc == SEIS_OK) rc = p->alloc(&gzd, (size_t)d.nx);
+    if (rc == SEIS_OK) rc = p->alloc(&ptab, (size_t)pad_tab_len(g.NX, g.NZ));
+    p->max_tab = std::max(p->max_tab, pad_tab_nx(g.NX) + pad_tab_nz(g.NZ) + 4);
     if (rc == SEIS_OK && (op == OP_RTM || op == OP_RTM_TRUE || op == OP_RTM_UPDOWN))
       rc = p->alloc(&g.strips, (size_t)d.nt * g.strip_len);
     if (rc == SEIS_OK && op == OP_RTM_UPDOWN) rc = p->alloc(&g.comp, 4 * (size_t)d.nx * d.nz);
@@ -478,7 +483,7 @@ int plan_create(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *descs
     }
     g.ntz = (g.NZ + shape_tz(p->shape) - 1) / shape_tz(p->shape);
     if (rc == SEIS_OK) {
-      g.vel = vel; g.dv = dv; g.wav = wav; g.rec = rec; g.gz = gzd;
+      g.vel = vel; g.dv = dv; g.wav = wav; g.rec = rec; g.gz = gzd; g.ptab = ptab;
       cudaError_t e = cudaMemcpyAsync(gzd, d.gz, sizeof(int) * d.nx, cudaMemcpyHostToDevice,
                                       ctx->stream);
       if (e != cudaSuccess) rc = fail(ctx, SEIS_ERR_CUDA, "gz upload: %s", cudaGetErrorString(e));
@@ -540,25 +545,38 @@ int plan_create(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *descs
 
 // Upload an unpadded [nx][nz] model of shot s into a padded device field.
 
-// One time step of every shot: the interior-tile kernel on the main stream and
-// the pad-tile kernel on the auxiliary stream, joined before the next step.
+// The absorbing coefficients of every shot's pad strips, from the velocities as
+// they are now; before the first step of a run.
+int pad_tabs(Plan &p) {
+  seis_fd_ctx *ctx = p.ctx;
+  CK(launch_pad_tab(p.d_sd, p.nshot, p.max_tab, ctx->stream));
+  ctx->launches++;
+  return SEIS_OK;
+}
+
+// One time step of every shot: all tiles in one launch, or the persistent
+// interior kernel on the main stream and the pad tiles on the auxiliary
+// stream, joined before the next step.
 int step(Plan &p, int mode, const StepArgs &a0, const ShotDev *shots = nullptr) {
   seis_fd_ctx *ctx = p.ctx;
   StepArgs a = a0;
   a.loop = p.loop;
+  const bool split = step_splits(mode, p.exact, p.n_int, p.shape, a.loop);
   cudaStream_t s_pad = ctx->stream;
-  if (p.overlap) {
+  if (split && p.overlap && p.n_pad > 0) {
     CK(cudaEventRecord(ctx->fork, ctx->stream));
     CK(cudaStreamWaitEvent(ctx->aux, ctx->fork, 0));
     s_pad = ctx->aux;
   }
+  if (split) a.pdl = 0;
+  a.maps = !shots || shots == p.d_sd ? p.d_maps : shots == p.d_sd_c ? p.d_maps_c : p.d_maps_h;
   CK(launch_step(mode, p.exact, shots ? shots : p.d_sd, p.d_tiles, p.n_int, p.n_pad, p.shape, a,
                  ctx->d_err, ctx->stream, s_pad));
-  if (p.overlap) {
+  if (s_pad != ctx->stream) {
     CK(cudaEventRecord(ctx->join, ctx->aux));
     CK(cudaStreamWaitEvent(ctx->stream, ctx->join, 0));
   }
-  ctx->launches += (p.n_int > 0) + (p.n_pad > 0);
+  ctx->launches += split ? 1 + (p.n_pad > 0) : 1;
   return SEIS_OK;
 }
 
@@ -708,6 +726,7 @@ int run_forward(Plan &p, int mode, const ShotDev *shots = nullptr) {
     a.illum_on = ill && it > p.ndel;  // fd.cpp:318, :763
     a.strip_k = (rtm && itp >= 0) ? itp : -1;
     a.snap_k = p.op == OP_BORN_ADJ ? snap_slot(it, p.NT - 1, p.snap_every) : -1;
+    a.pdl = it > 0;
     int rc = step(p, mode, a, shots);
     if (rc) return rc;
   }
@@ -845,7 +864,8 @@ int run_updown_reverse(Plan &p) {
 // (adjoint plans); reused by every later run until the velocity or the
 // wavelet changes.
 int source_pass(Plan &p) {
-  int rc = SEIS_OK;
+  int rc = pad_tabs(p);
+  if (rc) return rc;
   if (p.ck_every == 0) {
     rc = run_forward(p, MODE_MODEL);
   } else {
@@ -970,6 +990,7 @@ int run_adjoint(Plan &p) {
 // plan_run).
 int enqueue_operator(Plan &p) {
   int rc = clear_fields(p);
+  if (!rc) rc = pad_tabs(p);
   if (rc) return rc;
   switch (p.op) {
     case OP_MODEL: return run_forward(p, MODE_MODEL);
@@ -1331,14 +1352,15 @@ int time_steps(Plan &p, int steps, double *ms, double *bytes) {
     int64_t c = (int64_t)std::min(TX, g.NX - t.x0) * std::min(TZ, g.NZ - t.z0);
     ((int)i < n_int ? cells_int : cells_pad) += c;
   }
-  if (adj) {
-    int rc0 = edge_coefs(p);
+  {
+    int rc0 = adj ? edge_coefs(p) : pad_tabs(p);
     if (rc0) return rc0;
   }
   StepArgs a{};
   a.nshots = p.nshot;
   a.strip_k = -1;
   a.loop = p.loop;
+  a.maps = p.d_maps;
   // the interior tiles (the list's first n_int) or the pad tiles alone, on
   // the main / auxiliary stream
   auto launch = [&](bool interior) -> cudaError_t {

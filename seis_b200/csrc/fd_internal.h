@@ -47,25 +47,26 @@ struct Tile {
 // 2-D TMA tensor maps of one shot (each describes one margin-padded field
 // allocation, LDZ rows x ncols columns; box = staged rows x staged columns).
 // Pad tiles: wide boxes (TX + 2*HXC columns, TZ + 2*ZM rows) stage a field read
-// as "current"; narrow boxes (TX + 2 columns) a field read as "previous", the
-// velocity or dv.  Interior tiles: the current field with an HI-cell halo on
-// every side, the other arrays as the tile alone.
+// as "current"; a field read as "previous" has one column and four rows around
+// the tile (the adjoint's: narrow boxes, TX + 2 columns).  Interior tiles: the
+// current field with an HI-cell halo on every side, the other arrays as the
+// tile alone.
 enum MapIndex : int {
   MAP_FA_WIDE = 0,    // + rotating buffer index 0..2
-  MAP_FA_NARROW = 3,
-  MAP_FB_WIDE = 6,
-  MAP_FB_NARROW = 9,
-  MAP_VEL = 12,
-  MAP_DV = 13,
-  MAP_VEL_WIDE = 14,  // velocity with the wide halo (adjoint kernels)
-  MAP_FA_HALO = 15,   // interior tiles: (TX + 2 HI) x (TZ + 2 HI), + buffer index
-  MAP_FB_HALO = 18,
-  MAP_FA_TILE = 21,   // interior tiles: TX x TZ, + buffer index
-  MAP_FB_TILE = 24,
-  MAP_VEL_TILE = 27,
-  MAP_DV_TILE = 28,
-  MAP_VEL_HALO = 29,  // interior tiles of the adjoint: velocity with the HI-cell halo
-  NMAPS = 30,
+  MAP_FB_WIDE = 3,
+  MAP_FA_HALO = 6,    // interior tiles: (TX + 2 HI) x (TZ + 2 HI), + buffer index
+  MAP_FB_HALO = 9,
+  MAP_FA_PREV = 12,   // pad tiles: (TX + 2) x (TZ + 8), + buffer index
+  MAP_FB_PREV = 15,
+  MAP_FA_TILE = 18,   // interior tiles: TX x TZ, + buffer index
+  MAP_FB_TILE = 21,
+  MAP_VEL_TILE = 24,
+  MAP_DV_TILE = 25,
+  MAP_FA_NARROW = 26, // adjoint pad tiles, + buffer index
+  MAP_VEL_WIDE = 29,  // velocity with the wide halo (adjoint pad tiles)
+  MAP_VEL_HALO = 30,  // interior tiles of the adjoint: velocity with the HI-cell halo
+  MAP_VEL_PREV = 31,  // pad tiles: velocity, boxes as MAP_FA_PREV
+  NMAPS = 32,
 };
 
 // Device descriptor of one shot in a batch.  Scalars derived from dt/dx/dz are
@@ -122,7 +123,26 @@ struct ShotDev {
   // tap k of band cell i at edge_coef[k * edge_cells(NX, NZ) + i]; band
   // cells indexed by edge_index)
   float *edge_coef;
+  // absorbing coefficients of the pad strips (pad_tab_x, pad_tab_c), formed once per
+  // run from the velocity
+  const float *ptab;
 };
+// Layout of ptab.  The padded velocity repeats the model's edge cells
+// outward, so the one-way coefficients of a top or bottom strip depend on the
+// column alone, those of a left or right strip on the row alone and those of
+// a diagonal corner cell on the corner alone.  By row ([7][NZ rounded up to
+// whole tiles]): left a2, a3, rd, right a2, a3, rd, blend weight; by column
+// ([7][NX rounded up]): top a2, a3, rd, bottom a2, a3, rd, weight; then per
+// corner (2 right + bottom) a3, its quotient's divisor d and rd.  a2 = hdt2 / v,
+// a3 = v / 4 / h / h, rd = 1 / (a1 + a2) or 1 / d, stored as zero outside
+// [2^-30, 1].  Rows and columns beyond the grid repeat the last one.
+__host__ __device__ inline int pad_tab_nz(int NZ) { return (NZ + TZ_MAX - 1) / TZ_MAX * TZ_MAX; }
+__host__ __device__ inline int pad_tab_nx(int NX) { return (NX + TX_MAX - 1) / TX_MAX * TX_MAX; }
+__host__ __device__ inline int pad_tab_x(int NZ) { return 7 * pad_tab_nz(NZ); }  // by column
+__host__ __device__ inline int pad_tab_c(int NX, int NZ) {                      // [4][3]
+  return pad_tab_x(NZ) + 7 * pad_tab_nx(NX);
+}
+__host__ __device__ inline int pad_tab_len(int NX, int NZ) { return pad_tab_c(NX, NZ) + 12; }
 // Cells of the four edge bands of a padded grid: the 5 top and 5 bottom rows
 // (column-major, 5 rows per column) and the 5 left and 5 right columns.
 constexpr int EDGE_TAPS = 13;  // 7 along z (offsets -3..3), 6 along x (-3..3 but 0)
@@ -152,6 +172,10 @@ struct StepArgs {
   // interior kernel: -1 the persistent one when each of its CTAs gets at
   // least 4 tiles, else one tile per CTA; 0 one tile per CTA; 1 persistent
   int loop = -1;
+  // programmatic launch: the kernel may start before the last one on the
+  // stream (a step kernel of the same run) has finished
+  int pdl = 0;
+  const CUtensorMap *maps = nullptr;  // of the shot table: NMAPS per shot
 };
 
 // Allocation geometry of one field of a shot: LDZ floats per column, and the
@@ -188,13 +212,18 @@ enum StepMode : int {
 cudaError_t launch_step(int mode, bool exact, const ShotDev *d_shots, const Tile *d_tiles,
                         int n_int, int n_pad, int shape, const StepArgs &a, int *d_err,
                         cudaStream_t s_int, cudaStream_t s_pad);
+// Whether such a step is two launches (the persistent interior kernel and the
+// pad tiles), or one of all tiles.
+bool step_splits(int mode, bool exact, int n_int, int shape, int loop);
 namespace exact {
+bool step_splits(int mode, int n_int, int shape, int loop);
 cudaError_t launch_step(int mode, const ShotDev *d_shots, const Tile *d_tiles, int n_int,
                         int n_pad, int shape, const StepArgs &a, int *d_err, cudaStream_t s_int,
                         cudaStream_t s_pad);
 cudaError_t configure();
 }  // namespace exact
 namespace fast {
+bool step_splits(int mode, int n_int, int shape, int loop);
 cudaError_t launch_step(int mode, const ShotDev *d_shots, const Tile *d_tiles, int n_int,
                         int n_pad, int shape, const StepArgs &a, int *d_err, cudaStream_t s_int,
                         cudaStream_t s_pad);
@@ -209,6 +238,10 @@ cudaError_t launch_adjoint(int shape, const ShotDev *d_shots, const Tile *d_tile
                            cudaStream_t s_pad);
 cudaError_t configure_adjoint();
 }  // namespace fast
+// the absorbing coefficients of every shot's pad strips (ShotDev::ptab), after
+// its velocity is in place; max_len = the largest
+// pad_tab_nx + pad_tab_nz + 4 of the batch
+cudaError_t launch_pad_tab(const ShotDev *d_shots, int nshots, int max_len, cudaStream_t s);
 cudaError_t launch_finalize_image(const ShotDev *d_shots, int nshots, cudaStream_t s);
 
 // Vector operations of the CG solver (fd_vec.cu).  A dot product needs a

@@ -17,12 +17,9 @@ int LoopGrid<S, MODE>::ctas = 0;
 
 template <int S, int MODE>
 cudaError_t setup() {
-  cudaError_t e = cudaFuncSetAttribute(tile_kernel<S, MODE>,
+  cudaError_t e = cudaFuncSetAttribute(step_tile_kernel<S, MODE>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)TCfg<S, MODE>::bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(pad_tile_kernel<S, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)PCfg<S, MODE>::bytes);
+                                       (int)UCfg<S, MODE>::bytes);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(interior_loop_kernel<S, MODE>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -45,25 +42,43 @@ cudaError_t setup_shape() {
   return e;
 }
 
-// Interior tiles on s_int, pad tiles (one CTA each) on s_pad.  The interior
-// kernel is the persistent one as a.loop says; by default when each of its
-// CTAs gets at least LOOP_MIN_TILES tiles (its double buffering pays, and the
-// last round of tiles is a small part of the launch).
+// Every tile in one launch on s_int, or the interior tiles by the persistent
+// kernel on s_int and the pad tiles on s_pad: as `loop` says; by default the
+// latter when each persistent CTA gets at least LOOP_MIN_TILES tiles (its
+// double buffering pays, and the last round of tiles is a small part of the
+// launch).
 constexpr int LOOP_MIN_TILES = 4;
+template <int S, int MODE>
+bool splits(int n_int, int loop) {
+  return n_int > 0 && (loop > 0 || (loop < 0 && n_int >= LOOP_MIN_TILES * LoopGrid<S, MODE>::ctas));
+}
 template <int S, int MODE>
 cudaError_t launch_t(const ShotDev *d_shots, const Tile *d_tiles, int n_int, int n_pad,
                      const StepArgs &a, int *d_err, cudaStream_t s_int, cudaStream_t s_pad) {
   constexpr int NT = Geo<S>::NT;
-  const int G = LoopGrid<S, MODE>::ctas;
-  if (n_int > 0 && (a.loop > 0 || (a.loop < 0 && n_int >= LOOP_MIN_TILES * G))) {
+  const bool split = splits<S, MODE>(n_int, a.loop);
+  if (split) {
+    const int G = LoopGrid<S, MODE>::ctas;
     interior_loop_kernel<S, MODE><<<G < n_int ? G : n_int, NT, LCfg<S, MODE>::bytes, s_int>>>(
         d_shots, d_tiles, n_int, a, d_err);
-  } else if (n_int > 0) {
-    tile_kernel<S, MODE><<<n_int, NT, TCfg<S, MODE>::bytes, s_int>>>(d_shots, d_tiles, a, d_err);
+    d_tiles += n_int;
+    n_int = 0;
   }
-  if (n_pad > 0)
-    pad_tile_kernel<S, MODE><<<n_pad, NT, PCfg<S, MODE>::bytes, s_pad>>>(d_shots, d_tiles + n_int,
-                                                                       a, d_err);
+  if (n_int + n_pad > 0) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(n_int + n_pad);
+    c.blockDim = dim3(NT);
+    c.dynamicSmemBytes = UCfg<S, MODE>::bytes;
+    c.stream = n_int > 0 ? s_int : s_pad;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = a.pdl ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&c, step_tile_kernel<S, MODE>, d_shots, d_tiles, n_int,
+                                       n_pad, a, d_err);
+    if (e != cudaSuccess) return e;
+  }
   return cudaGetLastError();
 }
 
@@ -82,7 +97,24 @@ cudaError_t launch_mode(int mode, const ShotDev *d_shots, const Tile *d_tiles, i
       return cudaErrorInvalidValue;
   }
 }
+template <int S>
+bool splits_mode(int mode, int n_int, int loop) {
+  return mode == MODE_MODEL  ? splits<S, MODE_MODEL>(n_int, loop)
+         : mode == MODE_RCV ? splits<S, MODE_RCV>(n_int, loop)
+                            : splits<S, MODE_BORN>(n_int, loop);
+}
 }  // namespace
+
+bool step_splits(int mode, int n_int, int shape, int loop) {
+  switch (shape) {
+    case SHAPE_32x64: return splits_mode<SHAPE_32x64>(mode, n_int, loop);
+    case SHAPE_64x32: return splits_mode<SHAPE_64x32>(mode, n_int, loop);
+    case SHAPE_16x128: return splits_mode<SHAPE_16x128>(mode, n_int, loop);
+    case SHAPE_64x64: return splits_mode<SHAPE_64x64>(mode, n_int, loop);
+    case SHAPE_32x32: return splits_mode<SHAPE_32x32>(mode, n_int, loop);
+    default: return false;
+  }
+}
 
 cudaError_t configure() {
   cudaError_t e = setup_shape<SHAPE_32x64>();
