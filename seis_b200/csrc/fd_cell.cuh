@@ -31,19 +31,31 @@ __device__ __forceinline__ Coef coef(float v, const ShotDev &g) {
   return c;
 }
 
+// z + x y: rounded twice in the exact build, once in the contracted one (said
+// explicitly, so that the scalar and the packed forms of a formula agree)
+__device__ __forceinline__ float madd1(float x, float y, float z) {
+#ifdef SEIS_FAST_MATH
+  return __fmaf_rn(x, y, z);
+#else
+  return z + x * y;
+#endif
+}
 // sum_k a_k u[k] in the reference order (fd.cpp:1263-1268)
 __device__ __forceinline__ float lap8(float m4, float m3, float m2, float m1, float c, float p1,
                                       float p2, float p3, float p4) {
-  float s = m4 * SEIS_C0;
-  s = s + m3 * SEIS_C1;
-  s = s + m2 * SEIS_C2;
-  s = s + m1 * SEIS_C3;
-  s = s + c * SEIS_C4;
-  s = s + p1 * SEIS_C3;
-  s = s + p2 * SEIS_C2;
-  s = s + p3 * SEIS_C1;
-  s = s + p4 * SEIS_C0;
-  return s;
+  float s = __fmul_rn(m4, SEIS_C0);
+  s = madd1(m3, SEIS_C1, s);
+  s = madd1(m2, SEIS_C2, s);
+  s = madd1(m1, SEIS_C3, s);
+  s = madd1(c, SEIS_C4, s);
+  s = madd1(p1, SEIS_C3, s);
+  s = madd1(p2, SEIS_C2, s);
+  s = madd1(p3, SEIS_C1, s);
+  return madd1(p4, SEIS_C0, s);
+}
+// vz uzz + vx uxx + 2 c - p
+__device__ __forceinline__ float leapfrog(const Coef &k, float uzz, float uxx, float c, float p) {
+  return madd1(2.0f, c, madd1(k.vz, uzz, __fmul_rn(k.vx, uxx))) - p;
 }
 
 __device__ __forceinline__ float d2(float v, float k, float a, float b, float c) {
@@ -91,7 +103,7 @@ __device__ __forceinline__ float twoway_low(const A &cur, const AP &prev, float 
   const Coef k = coef(v, g);
   const float uzz = cur(ix, iz - 1) + cur(ix, iz + 1) - 2.0f * c;
   const float uxx = cur(ix + 1, iz) + cur(ix - 1, iz) - 2.0f * c;
-  return k.vz * uzz + k.vx * uxx + 2.0f * c - p;
+  return leapfrog(k, uzz, uxx, c, p);
 }
 
 // The same of a cell in the 8th-order region (modeling2D_high, :1259-1270).
@@ -104,7 +116,7 @@ __device__ __forceinline__ float twoway_high(const A &cur, const AP &prev, float
                          cur(ix, iz + 1), cur(ix, iz + 2), cur(ix, iz + 3), cur(ix, iz + 4));
   const float uxx = lap8(cur(ix - 4, iz), cur(ix - 3, iz), cur(ix - 2, iz), cur(ix - 1, iz), c,
                          cur(ix + 1, iz), cur(ix + 2, iz), cur(ix + 3, iz), cur(ix + 4, iz));
-  return k.vz * uzz + k.vx * uxx + 2.0f * c - p;
+  return leapfrog(k, uzz, uxx, c, p);
 }
 
 // One-way strip update, fd.cpp:1098-1104 (and the three mirrored strips).

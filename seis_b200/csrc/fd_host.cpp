@@ -348,14 +348,18 @@ int encode_maps(Plan &p, std::vector<ShotDev> &sds, CUtensorMap **d_out) {
     for (int k = 0; k < 3 && !rc; k++) {
       rc = encode_map(p.ctx, g, g.fa[k], rows, wide, &m[MAP_FA_WIDE + k]);
       if (!rc) rc = encode_map(p.ctx, g, g.fa[k], rows - 8, narrow, &m[MAP_FA_PREV + k]);
-      if (!rc && p.op == OP_BORN_ADJ)
-        rc = encode_map(p.ctx, g, g.fa[k], rows, narrow, &m[MAP_FA_NARROW + k]);
       if (!rc && g.fb[k]) rc = encode_map(p.ctx, g, g.fb[k], rows, wide, &m[MAP_FB_WIDE + k]);
       if (!rc && g.fb[k]) rc = encode_map(p.ctx, g, g.fb[k], rows - 8, narrow, &m[MAP_FB_PREV + k]);
     }
     if (!rc) rc = encode_map(p.ctx, g, g.vel, rows - 8, narrow, &m[MAP_VEL_PREV]);
-    if (!rc && p.op == OP_BORN_ADJ)
+    if (!rc && p.op == OP_BORN_ADJ) {
       rc = encode_map(p.ctx, g, g.vel, rows, wide, &m[MAP_VEL_WIDE]);
+      if (!rc)
+        rc = encode_map(p.ctx, g, g.vel, shape_tz(p.shape) + 2 * HI, shape_tx(p.shape) + 2 * HI,
+                        &m[MAP_VEL_HALO]);
+    }
+    for (int k = 0; k < 2 && !rc; k++)
+      if (g.adj_e[k]) rc = encode_map(p.ctx, g, g.adj_e[k], rows - 8, narrow, &m[MAP_E_PREV + k]);
     // interior tiles
     const int TX = shape_tx(p.shape), TZ = shape_tz(p.shape);
     for (int k = 0; k < 3 && !rc; k++) {
@@ -365,8 +369,6 @@ int encode_maps(Plan &p, std::vector<ShotDev> &sds, CUtensorMap **d_out) {
       if (!rc && g.fb[k]) rc = encode_map(p.ctx, g, g.fb[k], TZ, TX, &m[MAP_FB_TILE + k]);
     }
     if (!rc) rc = encode_map(p.ctx, g, g.vel, TZ, TX, &m[MAP_VEL_TILE]);
-    if (!rc && p.op == OP_BORN_ADJ)
-      rc = encode_map(p.ctx, g, g.vel, TZ + 2 * HI, TX + 2 * HI, &m[MAP_VEL_HALO]);
     if (!rc && g.dv) rc = encode_map(p.ctx, g, g.dv, TZ, TX, &m[MAP_DV_TILE]);
     if (rc) return rc;
   }
@@ -474,12 +476,13 @@ int plan_create(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *descs
                           op == OP_RTM_TRUE || op == OP_RTM_UPDOWN || op == OP_ILLUM_PLANE))
       rc = p->alloc(&g.img, (size_t)d.nx * d.nz);
     if (op == OP_ILLUM || op == OP_ILLUM_PLANE) g.illum = g.img;
-    if (rc == SEIS_OK && op == OP_BORN_ADJ) rc = p->alloc(&g.grad, (size_t)d.nx * d.nz);
+    if (rc == SEIS_OK && op == OP_BORN_ADJ) rc = p->alloc(&g.grad, (size_t)d.nx * image_ld(d.nz, d.pml));
     if (op == OP_BORN_ADJ) {
       if (rc == SEIS_OK) rc = alloc_field(*p, g, &g.adj_e[0]);
       if (rc == SEIS_OK) rc = alloc_field(*p, g, &g.adj_e[1]);
       if (rc == SEIS_OK) rc = alloc_field(*p, g, &g.adj_b);
       if (rc == SEIS_OK) rc = p->alloc(&g.edge_coef, (size_t)EDGE_TAPS * edge_cells(g.NX, g.NZ));
+      if (rc == SEIS_OK) rc = p->alloc(&g.atab, (size_t)adj_tab_len(g.NX, g.NZ));
     }
     g.ntz = (g.NZ + shape_tz(p->shape) - 1) / shape_tz(p->shape);
     if (rc == SEIS_OK) {
@@ -549,34 +552,39 @@ int plan_create(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *descs
 // they are now; before the first step of a run.
 int pad_tabs(Plan &p) {
   seis_fd_ctx *ctx = p.ctx;
-  CK(launch_pad_tab(p.d_sd, p.nshot, p.max_tab, ctx->stream));
+  CK(launch_pad_tab(p.exact, p.d_sd, p.nshot, p.max_tab,
+                    p.op == OP_BORN || p.op == OP_BORN_PLANE, ctx->stream));
   ctx->launches++;
   return SEIS_OK;
 }
 
 // One time step of every shot: all tiles in one launch, or the persistent
 // interior kernel on the main stream and the pad tiles on the auxiliary
-// stream, joined before the next step.
+// stream, joined before the next step.  MODE_ADJ runs over the adjoint's
+// tiles.
 int step(Plan &p, int mode, const StepArgs &a0, const ShotDev *shots = nullptr) {
   seis_fd_ctx *ctx = p.ctx;
   StepArgs a = a0;
   a.loop = p.loop;
-  const bool split = step_splits(mode, p.exact, p.n_int, p.shape, a.loop);
+  const bool adj = mode == MODE_ADJ, exact = p.exact && !adj;
+  const Tile *d_tiles = adj ? p.d_adj_tiles : p.d_tiles;
+  const int n_int = adj ? p.n_int_adj : p.n_int, n_pad = adj ? p.n_pad_adj : p.n_pad;
+  const bool split = step_splits(mode, exact, n_int, p.shape, a.loop);
   cudaStream_t s_pad = ctx->stream;
-  if (split && p.overlap && p.n_pad > 0) {
+  if (split && p.overlap && n_pad > 0) {
     CK(cudaEventRecord(ctx->fork, ctx->stream));
     CK(cudaStreamWaitEvent(ctx->aux, ctx->fork, 0));
     s_pad = ctx->aux;
   }
   if (split) a.pdl = 0;
   a.maps = !shots || shots == p.d_sd ? p.d_maps : shots == p.d_sd_c ? p.d_maps_c : p.d_maps_h;
-  CK(launch_step(mode, p.exact, shots ? shots : p.d_sd, p.d_tiles, p.n_int, p.n_pad, p.shape, a,
+  CK(launch_step(mode, exact, shots ? shots : p.d_sd, d_tiles, n_int, n_pad, p.shape, a,
                  ctx->d_err, ctx->stream, s_pad));
   if (s_pad != ctx->stream) {
     CK(cudaEventRecord(ctx->join, ctx->aux));
     CK(cudaStreamWaitEvent(ctx->stream, ctx->join, 0));
   }
-  ctx->launches += split ? 1 + (p.n_pad > 0) : 1;
+  ctx->launches += split ? 1 + (n_pad > 0) : 1;
   return SEIS_OK;
 }
 
@@ -653,7 +661,7 @@ int ensure_snapshots(Plan &p) {
     int nsnap = snap_slots(p, g.NT);
     int ntx = (g.NX + shape_tx(p.shape) - 1) / shape_tx(p.shape);
     unsigned char *snap = nullptr;
-    int rc = p.alloc(&snap, (size_t)nsnap * g.nx * g.nz * esize);
+    int rc = p.alloc(&snap, (size_t)nsnap * g.nx * image_ld(g.nz, g.pml) * esize);
     if (!rc) rc = p.alloc(&g.snap_scale, (size_t)nsnap * ntx * g.ntz);
     if (rc) return rc;
     g.snap = snap;
@@ -670,27 +678,6 @@ int ensure_snapshots(Plan &p) {
   return SEIS_OK;
 }
 
-// One reverse step of the exact adjoint over the adjoint tile list.
-int adj_step(Plan &p, const StepArgs &a0) {
-  seis_fd_ctx *ctx = p.ctx;
-  StepArgs a = a0;
-  a.loop = p.loop;
-  cudaStream_t s_pad = ctx->stream;
-  if (p.overlap) {
-    CK(cudaEventRecord(ctx->fork, ctx->stream));
-    CK(cudaStreamWaitEvent(ctx->aux, ctx->fork, 0));
-    s_pad = ctx->aux;
-  }
-  CK(fast::launch_adjoint(p.shape, p.d_sd, p.d_adj_tiles, p.n_int_adj, p.n_pad_adj, a,
-                          ctx->d_err, ctx->stream, s_pad));
-  if (p.overlap) {
-    CK(cudaEventRecord(ctx->join, ctx->aux));
-    CK(cudaStreamWaitEvent(ctx->stream, ctx->join, 0));
-  }
-  ctx->launches += (p.n_int_adj > 0) + (p.n_pad_adj > 0);
-  return SEIS_OK;
-}
-
 // Zero every wavefield buffer (margins included) and the images.
 int clear_fields(Plan &p) {
   seis_fd_ctx *ctx = p.ctx;
@@ -701,7 +688,7 @@ int clear_fields(Plan &p) {
       if (g.fb[k]) CK(cudaMemsetAsync(g.fb[k] - fg.origin, 0, sizeof(float) * fg.elems, ctx->stream));
     }
     if (g.img) CK(cudaMemsetAsync(g.img, 0, sizeof(float) * g.nx * g.nz, ctx->stream));
-    if (g.grad) CK(cudaMemsetAsync(g.grad, 0, sizeof(double) * g.nx * g.nz, ctx->stream));
+    if (g.grad) CK(cudaMemsetAsync(g.grad, 0, sizeof(double) * g.nx * image_ld(g.nz, g.pml), ctx->stream));
     if (g.comp) CK(cudaMemsetAsync(g.comp, 0, sizeof(float) * 4 * g.nx * g.nz, ctx->stream));
   }
   for (const ShotDev &g : p.sd_h) {
@@ -893,6 +880,7 @@ int source_pass(Plan &p) {
       a.rot = it;
       a.rot_b = it;
       a.src_k = it >= 1 ? it - 1 : -1;
+      a.pdl = it > 0 && it % p.ck_every != 0;
       rc = step(p, MODE_MODEL, a, p.d_sd_c);
     }
   }
@@ -926,27 +914,31 @@ int recompute_segment(Plan &p, int s0, int s1) {
     a.src_k = it >= 1 ? it - 1 : -1;
     const int sl = snap_slot(it, p.NT - 1, p.snap_every);
     a.snap_k = sl >= 0 ? sl - slot0 : -1;
+    a.pdl = it > s0;
     int rc = step(p, MODE_MODEL, a, p.d_sd_c);
     if (rc) return rc;
   }
   return SEIS_OK;
 }
 
-// Reverse pass of the exact adjoint: L_k for k = NT .. 0 from L_{k+1}, L_{k+2};
-// the step producing L_k images the source term of step k with mu(L_{k+1}).
-// The exact adjoint's edge-band coefficients of every shot of the plan.
-int edge_coefs(Plan &p) {
+// The exact adjoint's edge-band coefficients and strip tables of every shot.
+int adj_tables(Plan &p) {
   seis_fd_ctx *ctx = p.ctx;
-  int most = 0;
-  for (const ShotDev &g : p.sd) most = std::max(most, edge_cells(g.NX, g.NZ));
-  CK(fast::launch_edge_coef(p.d_sd, p.nshot, most, ctx->stream));
-  ctx->launches++;
+  int cells = 0, tab = 0;
+  for (const ShotDev &g : p.sd) {
+    cells = std::max(cells, edge_cells(g.NX, g.NZ));
+    tab = std::max(tab, adj_tab_nx(g.NX) + adj_tab_nz(g.NZ) + 4);
+  }
+  CK(fast::launch_adj_tables(p.d_sd, p.nshot, cells, tab, ctx->stream));
+  ctx->launches += 2;
   return SEIS_OK;
 }
 
+// Reverse pass of the exact adjoint: L_k for k = NT .. 0 from L_{k+1}, L_{k+2};
+// the step producing L_k images the source term of step k with mu(L_{k+1}).
 int run_adjoint(Plan &p) {
   seis_fd_ctx *ctx = p.ctx;
-  int rc0 = edge_coefs(p);
+  int rc0 = adj_tables(p);
   if (rc0) return rc0;
   for (const ShotDev &g : p.sd) {
     FieldGeom fg = field_geom(g.NX, g.NZ);
@@ -965,7 +957,9 @@ int run_adjoint(Plan &p) {
   const int C = p.ck_every > 0 ? p.ck_every : p.NT + 1;
   int slot0 = 0;
   for (int k = p.NT; k >= 0; k--, r++) {
+    bool fresh = false;  // the last launch was of the recomputed source field
     if (p.ck_every > 0 && k < p.NT && (k == p.NT - 1 || (k + 1) % C == 0)) {
+      fresh = true;
       const int s0 = (k / C) * C;
       int rc = recompute_segment(p, s0, k + 1);
       if (rc) return rc;
@@ -978,7 +972,8 @@ int run_adjoint(Plan &p) {
     const int sl = snap_slot(k, p.NT - 1, p.snap_every);
     a.snap_k = sl >= 0 ? sl - slot0 : -1;
     a.img_w = sl >= 0 ? snap_weight(k, p.NT - 1, p.snap_every) : 0.0f;
-    int rc = adj_step(p, a);
+    a.pdl = k < p.NT && !fresh;
+    int rc = step(p, MODE_ADJ, a);
     if (rc) return rc;
   }
   CK(launch_finalize_image(p.d_sd, p.nshot, ctx->stream));
@@ -1337,7 +1332,8 @@ namespace {
 int time_steps(Plan &p, int steps, double *ms, double *bytes) {
   seis_fd_ctx *ctx = p.ctx;
   const int TX = shape_tx(p.shape), TZ = shape_tz(p.shape);
-  int mode = p.op == OP_BORN ? MODE_BORN : MODE_MODEL;
+  const int mode = p.op == OP_BORN ? MODE_BORN : p.op == OP_BORN_ADJ ? MODE_ADJ : MODE_MODEL;
+  const bool exact = p.exact && mode != MODE_ADJ;
   int fields = p.op == OP_BORN ? 2 : 1;
   cudaEvent_t ev[5];
   for (auto &e : ev) CK(cudaEventCreate(&e));
@@ -1353,7 +1349,7 @@ int time_steps(Plan &p, int steps, double *ms, double *bytes) {
     ((int)i < n_int ? cells_int : cells_pad) += c;
   }
   {
-    int rc0 = adj ? edge_coefs(p) : pad_tabs(p);
+    int rc0 = adj ? adj_tables(p) : pad_tabs(p);
     if (rc0) return rc0;
   }
   StepArgs a{};
@@ -1366,10 +1362,8 @@ int time_steps(Plan &p, int steps, double *ms, double *bytes) {
   auto launch = [&](bool interior) -> cudaError_t {
     const int ni = interior ? n_int : 0, np = interior ? 0 : n_pad;
     const Tile *t0 = interior ? d_tl : d_tl + n_int;
-    return adj ? fast::launch_adjoint(p.shape, p.d_sd, t0, ni, np, a, ctx->d_err, ctx->stream,
-                                      ctx->aux)
-               : launch_step(mode, p.exact, p.d_sd, t0, ni, np, p.shape, a, ctx->d_err,
-                             ctx->stream, ctx->aux);
+    return launch_step(mode, exact, p.d_sd, t0, ni, np, p.shape, a, ctx->d_err, ctx->stream,
+                       ctx->aux);
   };
   double t_int = 0, t_pad = 0, t_step = 0;
   for (int k = 0; k < 2 * steps; k++) {
@@ -1389,17 +1383,13 @@ int time_steps(Plan &p, int steps, double *ms, double *bytes) {
       CK(cudaStreamWaitEvent(ctx->stream, ev[3], 0));
     } else if (p.overlap) {
       CK(cudaStreamWaitEvent(ctx->aux, ev[0], 0));
-      CK(adj ? fast::launch_adjoint(p.shape, p.d_sd, d_tl, n_int, n_pad, a, ctx->d_err,
-                                    ctx->stream, ctx->aux)
-             : launch_step(mode, p.exact, p.d_sd, d_tl, n_int, n_pad, p.shape, a, ctx->d_err,
-                           ctx->stream, ctx->aux));
+      CK(launch_step(mode, exact, p.d_sd, d_tl, n_int, n_pad, p.shape, a, ctx->d_err, ctx->stream,
+                     ctx->aux));
       CK(cudaEventRecord(ev[3], ctx->aux));
       CK(cudaStreamWaitEvent(ctx->stream, ev[3], 0));
     } else {
-      CK(adj ? fast::launch_adjoint(p.shape, p.d_sd, d_tl, n_int, n_pad, a, ctx->d_err,
-                                    ctx->stream, ctx->stream)
-             : launch_step(mode, p.exact, p.d_sd, d_tl, n_int, n_pad, p.shape, a, ctx->d_err,
-                           ctx->stream, ctx->stream));
+      CK(launch_step(mode, exact, p.d_sd, d_tl, n_int, n_pad, p.shape, a, ctx->d_err, ctx->stream,
+                     ctx->stream));
     }
     CK(cudaEventRecord(ev[4], ctx->stream));
     CK(cudaEventSynchronize(ev[4]));
@@ -1515,8 +1505,15 @@ int autotune(Plan &p, int steps, bool force, double *ms, int *best) {
       return apply(it->second);
     }
   }
-  int pick = 0;
-  double t_best = 0.0;
+  // An adjoint plan's shape is also the tiling of its 16-bit snapshots' scales,
+  // so a choice within the noise of the timing would change its results in
+  // their last bits from one process to the next: it stays at 64x32, at or
+  // near the fastest from a few hundred to a few thousand tiles (lead of the
+  // best of the others: at most 5% over 25 surveys), unless another shape
+  // leads by 8%.
+  const bool steady = p.op == OP_BORN_ADJ;
+  int pick = 0, pick_steady = 0;
+  double t_best = 0.0, t_steady = 0.0;
   for (int c = 0; c < 4 * NSHAPES; c++) {
     int rc = apply(c);
     double t[3];
@@ -1529,7 +1526,12 @@ int autotune(Plan &p, int steps, bool force, double *ms, int *best) {
       t_best = t[2];
       pick = c;
     }
+    if (s == SHAPE_64x32 && (t_steady == 0.0 || t[2] < t_steady)) {
+      t_steady = t[2];
+      pick_steady = c;
+    }
   }
+  if (steady && t_steady < 1.08 * t_best) pick = pick_steady;
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     g_tune_cache[key] = pick;

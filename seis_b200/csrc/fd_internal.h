@@ -48,7 +48,7 @@ struct Tile {
 // allocation, LDZ rows x ncols columns; box = staged rows x staged columns).
 // Pad tiles: wide boxes (TX + 2*HXC columns, TZ + 2*ZM rows) stage a field read
 // as "current"; a field read as "previous" has one column and four rows around
-// the tile (the adjoint's: narrow boxes, TX + 2 columns).  Interior tiles: the
+// the tile.  Interior tiles: the
 // current field with an HI-cell halo on every side, the other arrays as the
 // tile alone.
 enum MapIndex : int {
@@ -62,11 +62,11 @@ enum MapIndex : int {
   MAP_FB_TILE = 21,
   MAP_VEL_TILE = 24,
   MAP_DV_TILE = 25,
-  MAP_FA_NARROW = 26, // adjoint pad tiles, + buffer index
-  MAP_VEL_WIDE = 29,  // velocity with the wide halo (adjoint pad tiles)
-  MAP_VEL_HALO = 30,  // interior tiles of the adjoint: velocity with the HI-cell halo
-  MAP_VEL_PREV = 31,  // pad tiles: velocity, boxes as MAP_FA_PREV
-  NMAPS = 32,
+  MAP_VEL_PREV = 26,  // pad tiles: velocity, boxes as MAP_FA_PREV
+  MAP_E_PREV = 27,    // adjoint pad tiles: ring terms, + buffer index 0..1
+  MAP_VEL_WIDE = 29,  // adjoint pad tiles: velocity with the wide halo
+  MAP_VEL_HALO = 30,  // adjoint interior tiles: velocity with the HI-cell halo
+  NMAPS = 31,
 };
 
 // Device descriptor of one shot in a batch.  Scalars derived from dt/dx/dz are
@@ -96,11 +96,11 @@ struct ShotDev {
   float *img;            // image [nx][nz]
   const CUtensorMap *maps;  // NMAPS tensor maps of this shot (device memory)
   // source-term snapshots for the adjoint imaging condition: lap of the
-  // background field at every snap_every-th step, interior cells [nx][nz],
+  // background field at every snap_every-th step, model cells (image_index),
   // stored as snap_dtype with one power-of-two scale per (snapshot, tile)
   void *snap;
   float *snap_scale;     // [nsnap][ntile_x * ntile_z]
-  double *grad;          // FP64 imaging accumulator [nx][nz]
+  double *grad;          // FP64 imaging accumulator (image_index)
   int snap_dtype;        // SNAP_NONE / SNAP_F32 / SNAP_BF16 / SNAP_F16
   int snap_every;
   int ntz;               // tiles along z of this shot (scale indexing)
@@ -126,6 +126,8 @@ struct ShotDev {
   // absorbing coefficients of the pad strips (pad_tab_x, pad_tab_c), formed once per
   // run from the velocity
   const float *ptab;
+  // exact adjoint: the pad strips' transposed coefficients (adj_tab_kernel)
+  float *atab;
 };
 // Layout of ptab.  The padded velocity repeats the model's edge cells
 // outward, so the one-way coefficients of a top or bottom strip depend on the
@@ -135,7 +137,7 @@ struct ShotDev {
 // ([7][NX rounded up]): top a2, a3, rd, bottom a2, a3, rd, weight; then per
 // corner (2 right + bottom) a3, its quotient's divisor d and rd.  a2 = hdt2 / v,
 // a3 = v / 4 / h / h, rd = 1 / (a1 + a2) or 1 / d, stored as zero outside
-// [2^-30, 1].  Rows and columns beyond the grid repeat the last one.
+// [2^-30, 1]; the contracted build keeps a1 + a2 in the place of rd.  Rows and columns beyond the grid repeat the last one.
 __host__ __device__ inline int pad_tab_nz(int NZ) { return (NZ + TZ_MAX - 1) / TZ_MAX * TZ_MAX; }
 __host__ __device__ inline int pad_tab_nx(int NX) { return (NX + TX_MAX - 1) / TX_MAX * TX_MAX; }
 __host__ __device__ inline int pad_tab_x(int NZ) { return 7 * pad_tab_nz(NZ); }  // by column
@@ -143,6 +145,22 @@ __host__ __device__ inline int pad_tab_c(int NX, int NZ) {                      
   return pad_tab_x(NZ) + 7 * pad_tab_nx(NX);
 }
 __host__ __device__ inline int pad_tab_len(int NX, int NZ) { return pad_tab_c(NX, NZ) + 12; }
+// Layout of atab: by row [6][adj_tab_nz] (left, right), by column
+// [6][adj_tab_nx] (top, bottom), per corner [4][4]; row iz is entry iz + ADJ_TAB_M, columns alike.
+constexpr int ADJ_TAB_M = 4;
+__host__ __device__ inline int adj_tab_nz(int NZ) { return pad_tab_nz(NZ) + 2 * ADJ_TAB_M; }
+__host__ __device__ inline int adj_tab_nx(int NX) { return pad_tab_nx(NX) + 2 * ADJ_TAB_M; }
+__host__ __device__ inline int adj_tab_len(int NX, int NZ) {
+  return 6 * (adj_tab_nz(NZ) + adj_tab_nx(NX)) + 16;
+}
+// Layout of the snapshots and of the imaging accumulator: [nx][image_ld], rows
+// from the whole quad that holds the model's first row, so that every row quad
+// of a tile is one aligned vector.
+__host__ __device__ inline int image_ld(int nz, int pml) { return ((pml & 3) + nz + 3) / 4 * 4; }
+// model column x, padded row iz
+__host__ __device__ inline size_t image_index(int nz, int pml, int x, int iz) {
+  return (size_t)x * image_ld(nz, pml) + (size_t)(iz - (pml & ~3));
+}
 // Cells of the four edge bands of a padded grid: the 5 top and 5 bottom rows
 // (column-major, 5 rows per column) and the 5 left and 5 right columns.
 constexpr int EDGE_TAPS = 13;  // 7 along z (offsets -3..3), 6 along x (-3..3 but 0)
@@ -202,6 +220,7 @@ enum StepMode : int {
   MODE_MODEL = 0,    // field A; point source; record; optional strip save
   MODE_RCV = 1,      // field B; receiver injection rec*vt2 (reference RTM)
   MODE_BORN = 2,     // fields A (background) and B (scattered)
+  MODE_ADJ = 3,      // field A; reverse step of the exact Born adjoint (contracted build)
 };
 
 // One time step over every tile of a batch: the first n_int tiles are
@@ -216,6 +235,8 @@ cudaError_t launch_step(int mode, bool exact, const ShotDev *d_shots, const Tile
 // pad tiles), or one of all tiles.
 bool step_splits(int mode, bool exact, int n_int, int shape, int loop);
 namespace exact {
+cudaError_t launch_pad_tab(const ShotDev *d_shots, int nshots, int max_len, int born,
+                           cudaStream_t s);
 bool step_splits(int mode, int n_int, int shape, int loop);
 cudaError_t launch_step(int mode, const ShotDev *d_shots, const Tile *d_tiles, int n_int,
                         int n_pad, int shape, const StepArgs &a, int *d_err, cudaStream_t s_int,
@@ -223,25 +244,24 @@ cudaError_t launch_step(int mode, const ShotDev *d_shots, const Tile *d_tiles, i
 cudaError_t configure();
 }  // namespace exact
 namespace fast {
+cudaError_t launch_pad_tab(const ShotDev *d_shots, int nshots, int max_len, int born,
+                           cudaStream_t s);
 bool step_splits(int mode, int n_int, int shape, int loop);
 cudaError_t launch_step(int mode, const ShotDev *d_shots, const Tile *d_tiles, int n_int,
                         int n_pad, int shape, const StepArgs &a, int *d_err, cudaStream_t s_int,
                         cudaStream_t s_pad);
 cudaError_t configure();
-// one reverse step of the exact Born adjoint over the adjoint tile list
-// (interior tiles on s_int, pad tiles on s_pad)
-// the exact adjoint's edge-band coefficients of every shot (after its
-// velocity is in place); max_cells = the largest edge_cells of the batch
-cudaError_t launch_edge_coef(const ShotDev *d_shots, int nshots, int max_cells, cudaStream_t s);
-cudaError_t launch_adjoint(int shape, const ShotDev *d_shots, const Tile *d_tiles, int n_int,
-                           int n_pad, const StepArgs &a, int *d_err, cudaStream_t s_int,
-                           cudaStream_t s_pad);
-cudaError_t configure_adjoint();
+// the exact adjoint's edge-band coefficients and strip tables of every shot
+// (after its velocity is in place); max_cells = the largest edge_cells of the
+// batch, max_tab = the largest adj_tab_nx + adj_tab_nz + 4
+cudaError_t launch_adj_tables(const ShotDev *d_shots, int nshots, int max_cells, int max_tab,
+                              cudaStream_t s);
 }  // namespace fast
 // the absorbing coefficients of every shot's pad strips (ShotDev::ptab), after
 // its velocity is in place; max_len = the largest
-// pad_tab_nx + pad_tab_nz + 4 of the batch
-cudaError_t launch_pad_tab(const ShotDev *d_shots, int nshots, int max_len, cudaStream_t s);
+// pad_tab_nx + pad_tab_nz + 4 of the batch; born: for MODE_BORN steps
+cudaError_t launch_pad_tab(bool exact, const ShotDev *d_shots, int nshots, int max_len, int born,
+                           cudaStream_t s);
 cudaError_t launch_finalize_image(const ShotDev *d_shots, int nshots, cudaStream_t s);
 
 // Vector operations of the CG solver (fd_vec.cu).  A dot product needs a

@@ -37,60 +37,6 @@ __global__ void pad_kernel(const float *__restrict__ src, int nx, int nz, int pm
   }
 }
 
-// ptab of every shot: the coefficients of the one-way update (fd.cpp:1098-1104
-// and its mirrors, :1146-1178) and the blend weights (InitInversion.cpp:20-37),
-// each rounded as the reference rounds it.  Formed once per run: in the step
-// kernels these divisions cost more per pad cell than the stencil (the upper
-// left corner's, in double, held its whole tile for 15,000 cycles).
-__device__ float tab_recip(float d) {
-  const float r = 1.0f / d;
-  return r >= 0x1p-30f && r <= 1.0f ? r : 0.0f;
-}
-__device__ float tab_weight(int d, int pml) {
-  return d == 0 ? 1.0f : 1.0f - (float)d * 1.0f / (float)pml;
-}
-__global__ void pad_tab_kernel(const ShotDev *__restrict__ shots) {
-  const ShotDev &g = shots[blockIdx.y];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int NX = g.NX, NZ = g.NZ, n = pad_tab_nz(NZ), m = pad_tab_nx(NX);
-  float *T = const_cast<float *>(g.ptab);
-  if (i < n) {  // left and right strip of a row
-    const int iz = min(i, NZ - 1);
-    for (int b = 0; b < 2; b++) {
-      const float v = g.vel[(size_t)(b ? NX - 1 : 0) * g.LDZ + iz];
-      const float a2 = g.hdt2 / v;
-      float *t = T + 3 * b * n + i;
-      t[0] = a2;
-      t[n] = v / 4.0f / g.dz / g.dz;
-      t[2 * n] = tab_recip(g.a1x + a2);
-    }
-    T[6 * n + i] = tab_weight(max(max(g.pml - iz, iz - (g.pml + g.nz - 1)), 0), g.pml);
-  } else if (i < n + m) {  // top and bottom strip of a column
-    const int j = i - n, ix = min(j, NX - 1);
-    float *C = T + pad_tab_x(NZ);
-    for (int b = 0; b < 2; b++) {
-      const float v = g.vel[(size_t)ix * g.LDZ + (b ? NZ - 1 : 0)];
-      const float a2 = g.hdt2 / v;
-      float *t = C + 3 * b * m + j;
-      t[0] = a2;
-      t[m] = v / 4.0f / g.dx / g.dx;
-      t[2 * m] = tab_recip(g.a1z + a2);
-    }
-    C[6 * m + j] = tab_weight(max(max(g.pml - ix, ix - (g.pml + g.nx - 1)), 0), g.pml);
-  } else if (i < n + m + 4) {
-    const int c = i - n - m;
-    const float v = g.vel[(size_t)(c & 2 ? NX - 1 : 0) * g.LDZ + (c & 1 ? NZ - 1 : 0)];
-    // upper left: sqrt(2)/v/dt formed in double (:1176)
-    const float a3 = c == 0 ? __double2float_rn(g.sqrt2d / (double)v / (double)g.dt)
-                            : g.sqrt2f / v / g.dt;
-    const float d = g.ax1 + g.ax2 + a3;
-    float *t = T + pad_tab_c(NX, NZ) + 3 * c;
-    t[0] = a3;
-    t[1] = d;
-    t[2] = tab_recip(d);
-  }
-}
-
 __global__ void transpose_kernel(const float *__restrict__ src, int rows, int cols,
                                  float *__restrict__ dst) {
   __shared__ float tile[32][33];
@@ -291,7 +237,7 @@ __global__ void finalize_image_kernel(const ShotDev *__restrict__ shots) {
     float v = g.vel[(size_t)(x + g.pml) * g.LDZ + (z + g.pml)];
     float vt2 = coef(v, g).vt2;
     float vel3 = 2.0f / (v * v * v);
-    g.img[i] = (float)((double)(vt2 * vel3) * g.grad[i]);
+    g.img[i] = (float)((double)(vt2 * vel3) * g.grad[image_index(g.nz, g.pml, x, z + g.pml)]);
   }
 }
 
@@ -305,8 +251,7 @@ cudaError_t launch_finalize_image(const ShotDev *d_shots, int nshots, cudaStream
 
 cudaError_t configure_kernels() {
   cudaError_t e = exact::configure();
-  if (e == cudaSuccess) e = fast::configure();
-  return e == cudaSuccess ? fast::configure_adjoint() : e;
+  return e == cudaSuccess ? fast::configure() : e;
 }
 
 cudaError_t launch_step(int mode, bool use_exact, const ShotDev *d_shots, const Tile *d_tiles,
@@ -323,9 +268,10 @@ bool step_splits(int mode, bool use_exact, int n_int, int shape, int loop) {
                    : fast::step_splits(mode, n_int, shape, loop);
 }
 
-cudaError_t launch_pad_tab(const ShotDev *d_shots, int nshots, int max_len, cudaStream_t s) {
-  pad_tab_kernel<<<dim3((max_len + 127) / 128, nshots), 128, 0, s>>>(d_shots);
-  return cudaGetLastError();
+cudaError_t launch_pad_tab(bool use_exact, const ShotDev *d_shots, int nshots, int max_len,
+                           int born, cudaStream_t s) {
+  return use_exact ? exact::launch_pad_tab(d_shots, nshots, max_len, born, s)
+                   : fast::launch_pad_tab(d_shots, nshots, max_len, born, s);
 }
 
 cudaError_t launch_pad(const float *d_src, int nx, int nz, int pml, int LDZ, int clamp,

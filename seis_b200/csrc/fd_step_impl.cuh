@@ -6,6 +6,82 @@
 namespace seis {
 namespace SEIS_NS {
 
+// ptab of every shot: the coefficients of the one-way update (fd.cpp:1098-1104
+// and its mirrors, :1146-1178) and the blend weights (InitInversion.cpp:20-37),
+// each rounded as the build's per-cell formulas (absorb_geom) round it.  Formed once per run: in the step
+// kernels these divisions cost more per pad cell than the stencil (the upper
+// left corner's, in double, held its whole tile for 15,000 cycles).
+__device__ float tab_recip(float d) {
+  const float r = 1.0f / d;
+  return r >= 0x1p-30f && r <= 1.0f ? r : 0.0f;
+}
+// (the contracted build's Born steps have always rounded the ramp once, its
+// other steps twice)
+__device__ float tab_weight(int d, const ShotDev &g, int born) {
+#ifdef SEIS_FAST_MATH
+  return born ? __fmaf_rn(-(float)d, g.inv_pml, 1.0f) : 1.0f - __fmul_rn((float)d, g.inv_pml);
+#else
+  return d == 0 ? 1.0f : 1.0f - (float)d * 1.0f / (float)g.pml;
+#endif
+}
+__global__ void pad_tab_kernel(const ShotDev *__restrict__ shots, int born) {
+  const ShotDev &g = shots[blockIdx.y];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int NX = g.NX, NZ = g.NZ, n = pad_tab_nz(NZ), m = pad_tab_nx(NX);
+  float *T = const_cast<float *>(g.ptab);
+  if (i < n) {  // left and right strip of a row
+    const int iz = min(i, NZ - 1);
+    for (int b = 0; b < 2; b++) {
+      const float v = g.vel[(size_t)(b ? NX - 1 : 0) * g.LDZ + iz];
+#ifdef SEIS_FAST_MATH
+      const float a2 = g.hdt2 * (1.0f / v), a3 = v * g.q4dz2;
+#else
+      const float a2 = g.hdt2 / v, a3 = v / 4.0f / g.dz / g.dz;
+#endif
+      float *t = T + 3 * b * n + i;
+      t[0] = a2;
+      t[n] = a3;
+#ifdef SEIS_FAST_MATH
+      t[2 * n] = __fadd_rn(g.a1x, a2);
+#else
+      t[2 * n] = tab_recip(g.a1x + a2);
+#endif
+    }
+    T[6 * n + i] = tab_weight(max(max(g.pml - iz, iz - (g.pml + g.nz - 1)), 0), g, born);
+  } else if (i < n + m) {  // top and bottom strip of a column
+    const int j = i - n, ix = min(j, NX - 1);
+    float *C = T + pad_tab_x(NZ);
+    for (int b = 0; b < 2; b++) {
+      const float v = g.vel[(size_t)ix * g.LDZ + (b ? NZ - 1 : 0)];
+#ifdef SEIS_FAST_MATH
+      const float a2 = g.hdt2 * (1.0f / v), a3 = v * g.q4dx2;
+#else
+      const float a2 = g.hdt2 / v, a3 = v / 4.0f / g.dx / g.dx;
+#endif
+      float *t = C + 3 * b * m + j;
+      t[0] = a2;
+      t[m] = a3;
+#ifdef SEIS_FAST_MATH
+      t[2 * m] = __fadd_rn(g.a1z, a2);
+#else
+      t[2 * m] = tab_recip(g.a1z + a2);
+#endif
+    }
+    C[6 * m + j] = tab_weight(max(max(g.pml - ix, ix - (g.pml + g.nx - 1)), 0), g, born);
+  } else if (i < n + m + 4) {
+    const int c = i - n - m;
+    const float v = g.vel[(size_t)(c & 2 ? NX - 1 : 0) * g.LDZ + (c & 1 ? NZ - 1 : 0)];
+    // upper left: sqrt(2)/v/dt formed in double (:1176)
+    const float a3 = c == 0 ? __double2float_rn(g.sqrt2d / (double)v / (double)g.dt)
+                            : g.sqrt2f / v / g.dt;
+    const float d = g.ax1 + g.ax2 + a3;
+    float *t = T + pad_tab_c(NX, NZ) + 3 * c;
+    t[0] = a3;
+    t[1] = d;
+    t[2] = tab_recip(d);
+  }
+}
+
 namespace {
 // CTAs of the persistent interior kernel: as many as are resident at once
 template <int S, int MODE>
@@ -39,6 +115,9 @@ cudaError_t setup_shape() {
   cudaError_t e = setup<S, MODE_MODEL>();
   if (e == cudaSuccess) e = setup<S, MODE_RCV>();
   if (e == cudaSuccess) e = setup<S, MODE_BORN>();
+#ifdef SEIS_FAST_MATH
+  if (e == cudaSuccess) e = setup<S, MODE_ADJ>();
+#endif
   return e;
 }
 
@@ -93,12 +172,19 @@ cudaError_t launch_mode(int mode, const ShotDev *d_shots, const Tile *d_tiles, i
       return launch_t<S, MODE_RCV>(d_shots, d_tiles, n_int, n_pad, a, d_err, s_int, s_pad);
     case MODE_BORN:
       return launch_t<S, MODE_BORN>(d_shots, d_tiles, n_int, n_pad, a, d_err, s_int, s_pad);
+#ifdef SEIS_FAST_MATH
+    case MODE_ADJ:
+      return launch_t<S, MODE_ADJ>(d_shots, d_tiles, n_int, n_pad, a, d_err, s_int, s_pad);
+#endif
     default:
       return cudaErrorInvalidValue;
   }
 }
 template <int S>
 bool splits_mode(int mode, int n_int, int loop) {
+#ifdef SEIS_FAST_MATH
+  if (mode == MODE_ADJ) return splits<S, MODE_ADJ>(n_int, loop);
+#endif
   return mode == MODE_MODEL  ? splits<S, MODE_MODEL>(n_int, loop)
          : mode == MODE_RCV ? splits<S, MODE_RCV>(n_int, loop)
                             : splits<S, MODE_BORN>(n_int, loop);
@@ -114,6 +200,12 @@ bool step_splits(int mode, int n_int, int shape, int loop) {
     case SHAPE_32x32: return splits_mode<SHAPE_32x32>(mode, n_int, loop);
     default: return false;
   }
+}
+
+cudaError_t launch_pad_tab(const ShotDev *d_shots, int nshots, int max_len, int born,
+                           cudaStream_t s) {
+  pad_tab_kernel<<<dim3((max_len + 127) / 128, nshots), 128, 0, s>>>(d_shots, born);
+  return cudaGetLastError();
 }
 
 cudaError_t configure() {

@@ -184,13 +184,22 @@ __device__ __forceinline__ void save_strips(const ShotDev &g, int strip_k, int i
 // add, multiply and fused multiply-add of a pair are one instruction each and
 // round every element as the scalar operation does, so the issue slots of the
 // stencil's arithmetic halve and its results stay the same bits.
-// The exact build forms a product as x y + (-0), the zero read from constant
-// memory: the assembler contracts a packed multiply that feeds a packed add
-// into one fused operation whatever the rounding qualifiers and switches say,
-// and it cannot do that to a fused multiply-add of an unknown addend.
+//
+// The assembler contracts a packed multiply that feeds a packed add into one
+// fused operation, whatever the rounding qualifiers and switches say.  It
+// cannot do that to a fused multiply-add of an unknown addend: a product that
+// is rounded by itself (*) is x y + (-0), the zero read from constant memory;
+// what the contracted build fuses is written fused (madd, msub).
 struct V4 {
   float2 a, b;
 };
+__device__ __forceinline__ V4 v4(const float4 &q) {
+  return V4{make_float2(q.x, q.y), make_float2(q.z, q.w)};
+}
+__device__ __forceinline__ V4 v4(float x) { return V4{make_float2(x, x), make_float2(x, x)}; }
+__device__ __forceinline__ float4 f4(const V4 &v) {
+  return make_float4(v.a.x, v.a.y, v.b.x, v.b.y);
+}
 __device__ __forceinline__ uint64_t bits2(const float2 &x) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x.x), "f"(x.y));
@@ -206,11 +215,6 @@ __device__ __forceinline__ float2 add2(const float2 &x, const float2 &y) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(x)), "l"(bits2(y)));
   return pair2(r);
 }
-__device__ __forceinline__ float2 mul2(const float2 &x, const float2 &y) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(x)), "l"(bits2(y)));
-  return pair2(r);
-}
 __device__ __forceinline__ float2 fma2(const float2 &x, const float2 &y, const float2 &z) {
   uint64_t r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;"
@@ -218,34 +222,29 @@ __device__ __forceinline__ float2 fma2(const float2 &x, const float2 &y, const f
       : "l"(bits2(x)), "l"(bits2(y)), "l"(bits2(z)));
   return pair2(r);
 }
-__device__ __forceinline__ V4 v4(const float4 &q) {
-  return V4{make_float2(q.x, q.y), make_float2(q.z, q.w)};
-}
-__device__ __forceinline__ V4 v4(float x) { return V4{make_float2(x, x), make_float2(x, x)}; }
-__device__ __forceinline__ float4 f4(const V4 &v) {
-  return make_float4(v.a.x, v.a.y, v.b.x, v.b.y);
-}
+__constant__ float NEG_ZERO = -0.0f;
 __device__ __forceinline__ V4 operator+(const V4 &x, const V4 &y) {
   return V4{add2(x.a, y.a), add2(x.b, y.b)};
 }
-#ifndef SEIS_FAST_MATH
-__constant__ float NEG_ZERO = -0.0f;
-#endif
 __device__ __forceinline__ V4 operator*(const V4 &x, const V4 &y) {
-#ifdef SEIS_FAST_MATH
-  return V4{mul2(x.a, y.a), mul2(x.b, y.b)};
-#else
   const float2 z = make_float2(NEG_ZERO, NEG_ZERO);
   return V4{fma2(x.a, y.a, z), fma2(x.b, y.b, z)};
-#endif
 }
 __device__ __forceinline__ V4 operator*(const V4 &x, float y) { return x * v4(y); }
 __device__ __forceinline__ V4 fma4(const V4 &x, const V4 &y, const V4 &z) {
   return V4{fma2(x.a, y.a, z.a), fma2(x.b, y.b, z.b)};
 }
-// x - y: the product with -1 is exact
+// x - y, -x: the product with -1 is exact
 __device__ __forceinline__ V4 operator-(const V4 &x, const V4 &y) { return fma4(y, v4(-1.0f), x); }
-// z + x y: in the exact build rounded twice, as the reference's statement
+__device__ __forceinline__ V4 operator-(const V4 &x) { return x * v4(-1.0f); }
+__device__ __forceinline__ V4 operator/(const V4 &x, const V4 &y) {
+  return V4{make_float2(x.a.x / y.a.x, x.a.y / y.a.y), make_float2(x.b.x / y.b.x, x.b.y / y.b.y)};
+}
+// z + 2 x, z - 2 x: the doubling is exact, so the fused form rounds once as
+// the separate one does
+__device__ __forceinline__ V4 add_twice(const V4 &z, const V4 &x) { return fma4(x, v4(2.0f), z); }
+__device__ __forceinline__ V4 sub_twice(const V4 &z, const V4 &x) { return fma4(x, v4(-2.0f), z); }
+// z + x y and z - x y as the build rounds them
 __device__ __forceinline__ V4 madd(const V4 &x, const V4 &y, const V4 &z) {
 #ifdef SEIS_FAST_MATH
   return fma4(x, y, z);
@@ -254,18 +253,13 @@ __device__ __forceinline__ V4 madd(const V4 &x, const V4 &y, const V4 &z) {
 #endif
 }
 __device__ __forceinline__ V4 madd(const V4 &x, float y, const V4 &z) { return madd(x, v4(y), z); }
-// z - x y
 __device__ __forceinline__ V4 msub(const V4 &x, const V4 &y, const V4 &z) {
 #ifdef SEIS_FAST_MATH
-  return fma4(x * v4(-1.0f), y, z);
+  return fma4(-x, y, z);
 #else
   return z - x * y;
 #endif
 }
-// z + 2 x, z - 2 x: the doubling is exact, so the fused form rounds once as
-// the separate one does
-__device__ __forceinline__ V4 add_twice(const V4 &z, const V4 &x) { return fma4(x, v4(2.0f), z); }
-__device__ __forceinline__ V4 sub_twice(const V4 &z, const V4 &x) { return fma4(x, v4(-2.0f), z); }
 // rows one below / above a quad (e: the row after its last / before its first)
 __device__ __forceinline__ float4 shift_dn(const float4 &q, float e) {
   return make_float4(q.y, q.z, q.w, e);
@@ -310,23 +304,19 @@ __device__ __forceinline__ Coef4 coef4(const float4 &v, const ShotDev &g) {
   return c;
 }
 
-// Two-way update of two columns x 4 rows: u3 = vvzz uzz + vvxx uxx + 2 cur -
-// prev, 8th order (fd.cpp:1259-1270) and, for the rows of `low`, 2nd order
-// (:1226-1241); the current field from shared memory, the previous field and
-// the velocity in registers.  Shared-memory reads: 14 quads for 8 cells.
+// The second differences of two columns x 4 rows, 8th order (fd.cpp:1259-1268):
+// along z of the field CZ and along x of the field CX (the same one, except in
+// the adjoint), from shared memory: 14 quads for 8 cells.  `cen`: CX's quads.
 template <class SC>
-__device__ __forceinline__ void pair_twoway(const SC &C, const ShotDev &g, int ix, int iz0,
-                                            const float4 (&prv)[2], const float4 (&vel)[2],
-                                            float4 (&out)[2], float4 (&cen)[2],
-                                            unsigned low0 = 0u, unsigned low1 = 0u) {
+__device__ __forceinline__ void pair_sums(const SC &CZ, const SC &CX, int ix, int iz0, V4 (&uzz)[2],
+                                          V4 (&uxx)[2], float4 (&cen)[2]) {
   // both columns' sums along x as the window's ten columns go by: one quad of
   // it live at a time
   constexpr float W[9] = {SEIS_C0, SEIS_C1, SEIS_C2, SEIS_C3, SEIS_C4,
                           SEIS_C3, SEIS_C2, SEIS_C1, SEIS_C0};
-  V4 uxx[2];
 #pragma unroll
   for (int m = 0; m < 10; m++) {
-    const float4 q = C.quad(ix - 4 + m, iz0);
+    const float4 q = CX.quad(ix - 4 + m, iz0);
     const V4 x = v4(q);
     if (m == 0) uxx[0] = x * W[0];
     if (m == 1) uxx[1] = x * W[0];
@@ -336,16 +326,32 @@ __device__ __forceinline__ void pair_twoway(const SC &C, const ShotDev &g, int i
   }
 #pragma unroll
   for (int j = 0; j < 2; j++) {
-    const V4 uzz = lap8_along(C.quad(ix + j, iz0 - 4), cen[j], C.quad(ix + j, iz0 + 4));
+    const float4 zc = &CZ == &CX ? cen[j] : CZ.quad(ix + j, iz0);
+    uzz[j] = lap8_along(CZ.quad(ix + j, iz0 - 4), zc, CZ.quad(ix + j, iz0 + 4));
+  }
+}
+
+// Two-way update of two columns x 4 rows: u3 = vvzz uzz + vvxx uxx + 2 cur -
+// prev, 8th order (fd.cpp:1259-1270) and, for the rows of `low`, 2nd order
+// (:1226-1241); the previous field and the velocity in registers.
+template <class SC>
+__device__ __forceinline__ void pair_twoway(const SC &C, const ShotDev &g, int ix, int iz0,
+                                            const float4 (&prv)[2], const float4 (&vel)[2],
+                                            float4 (&out)[2], float4 (&cen)[2],
+                                            unsigned low0 = 0u, unsigned low1 = 0u) {
+  V4 uzz[2], uxx[2];
+  pair_sums(C, C, ix, iz0, uzz, uxx, cen);
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
     const Coef4 k = coef4(vel[j], g);
-    out[j] = f4(add_twice(madd(k.vx, uxx[j], k.vz * uzz), v4(cen[j])) - v4(prv[j]));
+    out[j] = f4(add_twice(madd(k.vz, uzz[j], k.vx * uxx[j]), v4(cen[j])) - v4(prv[j]));
     const unsigned low = j ? low1 : low0;
     if (low) {
       const V4 c = v4(cen[j]);
       const V4 lzz = sub_twice(v4(shift_up(cen[j], C(ix + j, iz0 - 1))) +
                                    v4(shift_dn(cen[j], C(ix + j, iz0 + 4))), c);
       const V4 lxx = sub_twice(v4(C.quad(ix + j + 1, iz0)) + v4(C.quad(ix + j - 1, iz0)), c);
-      const float4 l = f4(add_twice(madd(k.vx, lxx, k.vz * lzz), c) - v4(prv[j]));
+      const float4 l = f4(add_twice(madd(k.vz, lzz, k.vx * lxx), c) - v4(prv[j]));
 #pragma unroll
       for (int r = 0; r < 4; r++)
         if ((low >> r) & 1u) set_comp(out[j], r, comp(l, r));
@@ -353,6 +359,7 @@ __device__ __forceinline__ void pair_twoway(const SC &C, const ShotDev &g, int i
   }
 }
 
+#ifndef SEIS_FAST_MATH
 // x in [2^LO, 2^60] in magnitude
 template <int LO>
 __device__ __forceinline__ bool in_range(float x) {
@@ -366,16 +373,10 @@ __device__ __forceinline__ bool in_range(float x) {
 // overflows (1 <= d <= 2^30: from quotients of 2^-100 up); other quads (and
 // zero reciprocals, see ptab) divide.  Four quotients without a branch each:
 // the plain division tests every operand and takes its slow path for a zero
-// numerator, which is every pad cell that the wave has not reached.  The
-// contracted build keeps the product.
+// numerator, which is every pad cell that the wave has not reached.
 __device__ __forceinline__ float4 quot_quad(const V4 &n, const V4 &d, const V4 &rd) {
   const V4 q0 = n * rd;
   const float4 q = f4(q0), N = f4(n);
-#ifdef SEIS_FAST_MATH
-  const float4 D = f4(d), R = f4(rd);
-  if (R.x != 0.0f && R.y != 0.0f && R.z != 0.0f && R.w != 0.0f) return q;
-  return make_float4(N.x / D.x, N.y / D.y, N.z / D.z, N.w / D.w);
-#else
   if ((in_range<-100>(q.x) || N.x == 0.0f) && (in_range<-100>(q.y) || N.y == 0.0f) &&
       (in_range<-100>(q.z) || N.z == 0.0f) && (in_range<-100>(q.w) || N.w == 0.0f)) {
     const V4 m = d * -1.0f;
@@ -387,19 +388,21 @@ __device__ __forceinline__ float4 quot_quad(const V4 &n, const V4 &d, const V4 &
     if (N.w == 0.0f) r.w = N.w;
     return r;
   }
-  const float4 D = f4(d);
-  return make_float4(N.x / D.x, N.y / D.y, N.z / D.z, N.w / D.w);
-#endif
+  return f4(n / d);
 }
+#endif
 // 2 / x of four rows: the hardware's approximate reciprocal and two Newton
 // steps with fused residuals (Markstein, as above: correctly rounded; equal to
 // the division for every mantissa), doubled exactly.
+#ifndef SEIS_FAST_MATH
 __device__ __forceinline__ float rcp_approx(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
+#endif
 __device__ __forceinline__ V4 two_over(const V4 &x_) {
+#ifndef SEIS_FAST_MATH
   const float4 x = f4(x_);
   if (in_range<-60>(x.x) && in_range<-60>(x.y) && in_range<-60>(x.z) && in_range<-60>(x.w)) {
     const V4 m = x_ * -1.0f, one = v4(1.0f);
@@ -408,7 +411,8 @@ __device__ __forceinline__ V4 two_over(const V4 &x_) {
     y = fma4(fma4(m, y, one), y, y);
     return y + y;
   }
-  return v4(make_float4(2.0f / x.x, 2.0f / x.y, 2.0f / x.z, 2.0f / x.w));
+#endif
+  return v4(2.0f) / x_;
 }
 
 // Second time difference of the background field over dt^2 (fd.cpp:134-139)
@@ -428,53 +432,65 @@ __device__ __forceinline__ float4 ldg4(const float *p) {
 }
 
 // Write this thread's source-term values (lap of the background field) of
-// snapshot `k`: cells (xs[i], zs[i]) where bit i of `mask` is set.  BF16 / FP16
-// snapshots carry one power-of-two scale per (snapshot, tile), taken from the
-// tile's largest magnitude so that the scaled values lie in [0.5, 1).  Every
-// thread of the CTA calls this (it holds block barriers).
-template <int NTH, int NV, int TX, int TZ>
-__device__ void snap_write(const ShotDev &g, int k, int x0, int z0, const float (&v)[NV],
-                           const int (&xs)[NV], const int (&zs)[NV], unsigned mask, float *red) {
+// snapshot `k`: two column quads (columns ix, ix + 1 from row iz0), the rows of
+// mask[j], zero in a quad's other rows.  BF16 / FP16 snapshots carry one
+// power-of-two scale per (snapshot, tile), taken from the tile's largest
+// magnitude so that the scaled values lie in [0.5, 1).  Every thread of the CTA
+// calls this (it holds block barriers).
+template <int NTH, int TX, int TZ>
+__device__ __forceinline__ void snap_write(const ShotDev &g, int k, int x0, int z0, int ix, int iz0,
+                                           float4 (&v)[2], const unsigned (&mask)[2], float *red) {
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+      if (!((mask[j] >> r) & 1u)) set_comp(v[j], r, 0.0f);
   float scale = 1.0f;
   if (g.snap_dtype != SNAP_F32) {
     float m = 0.0f;
 #pragma unroll
-    for (int i = 0; i < NV; i++)
-      if ((mask >> i) & 1u) m = fmaxf(m, fabsf(v[i]));
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+      for (int r = 0; r < 4; r++) m = fmaxf(m, fabsf(comp(v[j], r)));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) red[warp] = m;
     __syncthreads();
-    if (warp == 0) {
-      m = lane < NTH / 32 ? red[lane] : 0.0f;
+    m = 0.0f;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-      if (lane == 0) {
-        int e = 0;
-        frexpf(m, &e);
-        // tiny (denormal) maxima would overflow the scale: clamp to 2^126
-        float sc = m > 0.0f ? ldexpf(1.0f, min(-e, 126)) : 1.0f;
-        red[32] = sc;
-        const int ntx = (g.NX + TX - 1) / TX;
-        g.snap_scale[(size_t)k * ntx * g.ntz + (x0 / TX) * g.ntz + z0 / TZ] = sc;
-      }
+    for (int w = 0; w < NTH / 32; w++) m = fmaxf(m, red[w]);
+    int e = 0;
+    frexpf(m, &e);
+    // tiny (denormal) maxima would overflow the scale: clamp to 2^126
+    scale = m > 0.0f ? ldexpf(1.0f, min(-e, 126)) : 1.0f;
+    if (threadIdx.x == 0) {
+      const int ntx = (g.NX + TX - 1) / TX;
+      g.snap_scale[(size_t)k * ntx * g.ntz + (x0 / TX) * g.ntz + z0 / TZ] = scale;
     }
     __syncthreads();
-    scale = red[32];
   }
-  const size_t base = (size_t)k * g.nx * g.nz;
+  const size_t base = (size_t)k * g.nx * image_ld(g.nz, g.pml);
 #pragma unroll
-  for (int i = 0; i < NV; i++) {
-    if (!((mask >> i) & 1u)) continue;
-    const size_t idx = base + (size_t)(xs[i] - g.pml) * g.nz + (zs[i] - g.pml);
-    const float q = v[i] * scale;
-    if (g.snap_dtype == SNAP_F32)
-      reinterpret_cast<float *>(g.snap)[idx] = q;
-    else if (g.snap_dtype == SNAP_BF16)
-      reinterpret_cast<__nv_bfloat16 *>(g.snap)[idx] = __float2bfloat16_rn(q);
-    else
-      reinterpret_cast<__half *>(g.snap)[idx] = __float2half_rn(q);
+  for (int j = 0; j < 2; j++) {
+    if (!mask[j]) continue;
+    const size_t i = base + image_index(g.nz, g.pml, ix + j - g.pml, iz0);
+    const float4 q = make_float4(v[j].x * scale, v[j].y * scale, v[j].z * scale, v[j].w * scale);
+    if (g.snap_dtype == SNAP_F32) {
+      *reinterpret_cast<float4 *>(reinterpret_cast<float *>(g.snap) + i) = q;
+    } else {
+      uint2 h;
+      if (g.snap_dtype == SNAP_BF16) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(q.x, q.y), hi = __floats2bfloat162_rn(q.z, q.w);
+        h.x = *reinterpret_cast<const uint32_t *>(&lo);
+        h.y = *reinterpret_cast<const uint32_t *>(&hi);
+      } else {
+        const __half2 lo = __floats2half2_rn(q.x, q.y), hi = __floats2half2_rn(q.z, q.w);
+        h.x = *reinterpret_cast<const uint32_t *>(&lo);
+        h.y = *reinterpret_cast<const uint32_t *>(&hi);
+      }
+      *reinterpret_cast<uint2 *>(reinterpret_cast<unsigned short *>(g.snap) + i) = h;
+    }
   }
 }
 
@@ -572,8 +588,9 @@ __device__ __forceinline__ void halo_cell(int i, int x0, int z0, int &hx, int &h
   }
 }
 
-// Pad quads of a tile: the columns' row quads [4q, 4q + 3] that hold at least
-// one pad cell of the grid, enumerated column by column, rows fastest (see
+// Row quads [4q, 4q + 3] of a tile's columns that hold at least one grid cell
+// outside a rectangle [rx0, rx1) x [rz0, rz1) (the model, or the model less its
+// edge cells), enumerated column by column, rows fastest (see
 // CellList).
 struct QuadList {
   int x0, xe;      // tile columns inside the grid
@@ -581,14 +598,14 @@ struct QuadList {
   int top, bot;    // quads of such a column from the top / from the bottom
   int cp, cm, n;   // quads per other column, per crossing column, in all
   float rcp, rcm;
-  __device__ __forceinline__ QuadList(int x0_, int z0, int xe_, int ze, const ShotDev &g)
+  __device__ __forceinline__ QuadList(int x0_, int z0, int xe_, int ze, int rx0, int rx1, int rz0,
+                                      int rz1)
       : x0(x0_), xe(xe_) {
-    ma = min(max(g.pml, x0), xe);
-    mb = min(max(g.pml + g.nx, ma), xe);
+    ma = min(max(rx0, x0), xe);
+    mb = min(max(rx1, ma), xe);
     cp = (ze - z0 + 3) / 4;
-    top = min(max(0, (min(ze, g.pml) - z0 + 3) / 4), cp);
-    const int zb = g.pml + g.nz;  // first row below the model
-    bot = zb < ze ? cp - max(0, zb - z0) / 4 : 0;
+    top = min(max(0, (min(ze, rz0) - z0 + 3) / 4), cp);
+    bot = rz1 < ze ? cp - max(0, rz1 - z0) / 4 : 0;
     if (top + bot > cp) top = cp, bot = 0;
     cm = top + bot;
     n = (xe - x0 - (mb - ma)) * cp + (mb - ma) * cm;
@@ -627,11 +644,14 @@ __device__ __forceinline__ float4 oneway_quad(float a1, const V4 &a2, const V4 &
                                               const float4 &pi_, const float4 &ptp,
                                               const float4 &ptm) {
   const V4 u3i = v4(u3i_), pK = v4(pK_), pi = v4(pi_), A1 = v4(a1);
-  V4 t = u3i * (-a1);
-  t = msub(A1, pK - pi, t);
+  V4 t = madd(u3i, v4(-a1), (pK - pi) * (-a1));
   t = madd(a2, sub_twice(sub_twice(pK, v4(cK)) + u3i + pi, v4(ci)), t);
   t = msub(a3, sub_twice(sub_twice(v4(u3tp) + v4(u3tm), u3i) + v4(ptp) + v4(ptm), pK), t);
-  return quot_quad(t * -1.0f, A1 + a2, rd);
+#ifdef SEIS_FAST_MATH
+  return f4(-t / rd);  // rd: the table's a1 + a2
+#else
+  return quot_quad(-t, A1 + a2, rd);
+#endif
 }
 
 // A tile's part of ptab in shared memory.
@@ -733,14 +753,26 @@ __device__ __forceinline__ float4 absorb_quad(const PadQuad &q, const TileTab<TX
     const int r = __ffs(q.c) - 1, iz = iz0 + r;
     const float *t = T.c[2 * (q.sx < 0) + (q.sz < 0)];
     const float n = -(-g.ax1 * U(cx, iz + q.sz) - g.ax2 * U(cx + q.sx, iz) + t[0] * (-C(cx, iz)));
+#ifdef SEIS_FAST_MATH
+    const float s = n / t[1];
+#else
     const float s = quot_quad(v4(n), v4(t[1]), v4(t[2])).x;
+#endif
 #pragma unroll
     for (int k = 0; k < 4; k++)
       if (k == r) set_comp(o, k, s);
   }
   const V4 w = q.xw ? v4(T.wx[col]) : v4(*reinterpret_cast<const float4 *>(&T.wz[row]));
-  return f4(madd(v4(o), v4(1.0f) - w, v4(u) * w));
+  return f4(madd(v4(u), w, v4(o) * (v4(1.0f) - w)));
 }
+
+template <int S, int MODE>
+struct UCfg;
+}  // namespace SEIS_NS
+}  // namespace seis
+#include "fd_adjoint.cuh"
+namespace seis {
+namespace SEIS_NS {
 
 // Staged arrays of one tile of the one-tile-per-CTA kernel.  Pad tiles: the
 // current fields with the wide halo, the previous fields and the velocity with
@@ -760,19 +792,27 @@ struct UCfg {
   static constexpr int CUR = align32(G::CW_C * G::SR);
   static constexpr int PRV = align32(G::CW_P * PR);
   static constexpr int U3 = align32(G::U3N);
-  static constexpr int DV = BORN ? G::TX * G::TZ : 0;
-  static constexpr int TAB = align32(TileTab<G::TX, G::TZ>::BYTES / 4);
+  static constexpr bool ADJ = MODE == MODE_ADJ;
+  // the velocity (adjoint: with the current field's halo) and, in the
+  // adjoint, the second weighted field; Born: the perturbation; adjoint: the
+  // ring terms (pad tiles)
+  static constexpr int VEL = ADJ ? CUR : PRV, WGT = ADJ ? CUR : 0;
+  static constexpr int DV = BORN ? G::TX * G::TZ : ADJ ? PRV : 0;
+  static constexpr int TAB_BYTES = ADJ ? AdjTab<G::TX, G::TZ>::BYTES : TileTab<G::TX, G::TZ>::BYTES;
+  static constexpr int TAB = align32(TAB_BYTES / 4);
   // interior tiles
   static constexpr int CW = G::TX + 2 * HI, RW = G::TZ + 2 * HI;
   static constexpr int CUR_I = align32(CW * RW), PRV_I = G::TX * G::TZ;
   // offsets: current fields, previous fields, velocity, perturbation, table,
   // two-way values
-  static constexpr int O_P = NF * CUR, O_V = O_P + NF * PRV, O_D = O_V + PRV, O_T = O_D + DV;
+  static constexpr int O_P = NF * CUR, O_V = O_P + NF * PRV, O_W = O_V + VEL;
+  static constexpr int O_D = O_W + WGT, O_T = O_D + DV;
   static constexpr int O_U = O_T + TAB, FLOATS = O_U + NF * U3;
   static_assert(CUR_I <= CUR && PRV_I <= PRV, "an interior tile fits a pad tile's memory");
   static constexpr size_t bytes = sizeof(float) * (size_t)FLOATS + 2 * sizeof(uint64_t);
-  static constexpr int TX_PAD = (NF * G::CW_C * G::SR + (NF + 1) * G::CW_P * PR + DV) * 4;
-  static constexpr int TX_INT = (NF * CW * RW + (NF + 1) * PRV_I + DV) * 4;
+  static constexpr int TX_PAD = ((NF + ADJ) * G::CW_C * G::SR + (NF + 1) * G::CW_P * PR +
+                                 (BORN ? DV : 0)) * 4;
+  static constexpr int TX_INT = ((NF + ADJ) * CW * RW + (NF + !ADJ) * PRV_I + (BORN ? DV : 0)) * 4;
   // at most 768 threads per SM (85 registers a thread; at 64 they spill and
   // one field measured 5% slower, at 128 up to 20% slower)
   static constexpr int CAP = 768 / G::NT;
@@ -873,15 +913,8 @@ __device__ __forceinline__ void interior_cells(const ShotDev &g, const StepArgs 
     }
   }
   if (snap) {
-    float lv[8];
-    int lx[8], lz[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      lv[k] = comp(lap[k / 4], k % 4);
-      lx[k] = ix + k / 4;
-      lz[k] = iz0 + k % 4;
-    }
-    snap_write<NT_T, 8, TX, TZ>(g, aa.snap_k, x0, z0, lv, lx, lz, 0xFFu, red);
+    const unsigned all[2] = {0xFu, 0xFu};
+    snap_write<NT_T, TX, TZ>(g, aa.snap_k, x0, z0, ix, iz0, lap, all, red);
   }
 }
 
@@ -1084,17 +1117,7 @@ __device__ __forceinline__ bool pad_cells(const ShotDev &g, const StepArgs &a, i
   }
 
   // snapshot of the model cells' source terms (holds block barriers)
-  if (snap) {
-    float lv[8];
-    int lx[8], lz[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      lv[k] = comp(lap[k / 4], k % 4);
-      lx[k] = ix + k / 4;
-      lz[k] = iz0 + k % 4;
-    }
-    snap_write<NT_T, 8, TX, TZ>(g, aa.snap_k, x0, z0, lv, lx, lz, cm[0] | cm[1] << 4, red);
-  }
+  if (snap) snap_write<NT_T, TX, TZ>(g, aa.snap_k, x0, z0, ix, iz0, lap, cm, red);
 
   // 3. the halo ring: the same two-way values, injection and scattering
   // source, for the halo cells next to a pad cell of the tile (the one-way
@@ -1147,7 +1170,7 @@ __device__ __forceinline__ bool pad_cells(const ShotDev &g, const StepArgs &a, i
   __syncthreads();
 
   // 4. pad quads: one-way update and blend, shared evenly by all threads
-  const QuadList pads(x0, z0, xe, ze, g);
+  const QuadList pads(x0, z0, xe, ze, g.pml, g.pml + g.nx, g.pml, g.pml + g.nz);
   for (int i = tid; i < pads.n; i += NT_T) {
     int cx, dz;
     pads.quad(i, cx, dz);
@@ -1231,8 +1254,12 @@ __global__ void __launch_bounds__(Geo<S>::NT, UCfg<S, MODE>::MIN_CTAS) step_tile
     mbar_expect_tx(bar, (uint32_t)(pad ? K::TX_PAD : K::TX_INT));
     const int xc = pad ? xt - HXC : xt - HI, zc = pad ? t.z0 : zt - HI;
     const int xp = pad ? xt - 1 : xt, zp = pad ? zt - 4 : zt;
-    tma_load_2d(sm + K::O_V, m + (pad ? MAP_VEL_PREV : MAP_VEL_TILE), zp, xp, bar);
+    if (K::ADJ)
+      tma_load_2d(sm + K::O_V, m + (pad ? MAP_VEL_WIDE : MAP_VEL_HALO), zc, xc, bar);
+    else
+      tma_load_2d(sm + K::O_V, m + (pad ? MAP_VEL_PREV : MAP_VEL_TILE), zp, xp, bar);
     if (BORN) tma_load_2d(sm + K::O_D, m + MAP_DV_TILE, zt, xt, bar);
+    if (K::ADJ && pad) prefetch_map(m + MAP_E_PREV + (a.rot & 1));
     pdl_wait();
     tma_load_2d(sm, mc, zc, xc, bar);
     tma_load_2d(sm + K::O_P, mp, zp, xp, bar);
@@ -1240,9 +1267,13 @@ __global__ void __launch_bounds__(Geo<S>::NT, UCfg<S, MODE>::MIN_CTAS) step_tile
       tma_load_2d(sm + K::CUR, mcb, zc, xc, bar);
       tma_load_2d(sm + K::O_P + K::PRV, mpb, zp, xp, bar);
     }
+    if (K::ADJ && pad) tma_load_2d(sm + K::O_D, m + MAP_E_PREV + (a.rot & 1), zp, xp, bar);
     if (pad) {  // needed last, and its address takes one more read
-      mbar_expect_tx(bar + 1, (uint32_t)TileTab<TX, TZ>::BYTES);
-      reinterpret_cast<TileTab<TX, TZ> *>(sm + K::O_T)->issue(shots[t.shot], t.x0, t.z0, bar + 1);
+      mbar_expect_tx(bar + 1, (uint32_t)K::TAB_BYTES);
+      if (K::ADJ)
+        reinterpret_cast<AdjTab<TX, TZ> *>(sm + K::O_T)->issue(shots[t.shot], t.x0, t.z0, bar + 1);
+      else
+        reinterpret_cast<TileTab<TX, TZ> *>(sm + K::O_T)->issue(shots[t.shot], t.x0, t.z0, bar + 1);
     }
   } else {
     for (int i = tid; i < (int)(sizeof(ShotDev) / sizeof(int)); i += NT_T - 32)
@@ -1259,20 +1290,30 @@ __global__ void __launch_bounds__(Geo<S>::NT, UCfg<S, MODE>::MIN_CTAS) step_tile
     gzq[j] = x >= 0 && x < g.nx ? g.gz[x] + g.pml : -1;
   }
   pdl_wait();
+  Imager im;
+  if (K::ADJ) im.template load<TX, TZ>(g, a, t.x0, t.z0, ix, iz0);
   if (!mbar_wait(bar, 0)) {
     if (tid == 0) atomicExch(err, 1);
     return;
   }
   if (pad) {
-    if (!pad_cells<S, MODE>(g, a, t.x0, t.z0, sm, bar + 1, gzq, red) && tid == 0)
-      atomicExch(err, 1);
+    bool ok;
+    if constexpr (K::ADJ)
+      ok = adj_pad_cells<S>(g, a, t.x0, t.z0, sm, bar + 1, gzq, im);
+    else
+      ok = pad_cells<S, MODE>(g, a, t.x0, t.z0, sm, bar + 1, gzq, red);
+    if (!ok && tid == 0) atomicExch(err, 1);
   } else {
     using SW = SAT<K::RW>;
     using ST = SAT<TZ>;
     const SW CA{sm, t.x0 - HI, t.z0 - HI}, CB{sm + (NF - 1) * K::CUR, t.x0 - HI, t.z0 - HI};
     const ST PA{sm + K::O_P, t.x0, t.z0}, PB{sm + K::O_P + (NF - 1) * K::PRV, t.x0, t.z0};
-    const ST V{sm + K::O_V, t.x0, t.z0}, D{sm + K::O_D, t.x0, t.z0};
-    interior_cells<S, MODE>(g, a, t.x0, t.z0, CA, CB, PA, PB, V, D, gzq, red);
+    if constexpr (K::ADJ) {
+      adj_interior_cells<S>(g, a, t.x0, t.z0, sm, sm + K::O_V, sm + K::O_W, PA, gzq, im);
+    } else {
+      const ST V{sm + K::O_V, t.x0, t.z0}, D{sm + K::O_D, t.x0, t.z0};
+      interior_cells<S, MODE>(g, a, t.x0, t.z0, CA, CB, PA, PB, V, D, gzq, red);
+    }
   }
 }
 
@@ -1285,17 +1326,20 @@ template <int S, int MODE>
 struct LCfg {
   using G = Geo<S>;
   static constexpr bool BORN = MODE == MODE_BORN;
-  static constexpr int NCUR = BORN ? 2 : 1;  // current fields
-  static constexpr int NOTH = BORN ? 4 : 2;  // prev, vel [, prev B, dv]
+  static constexpr bool ADJ = MODE == MODE_ADJ;
+  static constexpr int NCUR = BORN || ADJ ? 2 : 1;  // current fields; adjoint: field, velocity
+  static constexpr int NOTH = BORN ? 4 : ADJ ? 1 : 2;  // prev, vel [, prev B, dv]; adjoint: prev
   static constexpr int CW = G::TX + 2 * HI, RW = G::TZ + 2 * HI;
   static constexpr int TILE = G::TX * G::TZ;
   static constexpr int STAGE = NCUR * CW * RW + NOTH * TILE;  // floats
-  static constexpr size_t bytes = 2 * sizeof(float) * (size_t)STAGE + 2 * sizeof(uint64_t);
+  static constexpr int WGT = ADJ ? CW * RW : 0;  // the second weighted field
+  static constexpr size_t bytes =
+      sizeof(float) * (2 * (size_t)STAGE + WGT) + 2 * sizeof(uint64_t);
   // static shared memory: two shot tables and the snapshot reduction
   static constexpr size_t static_bytes = 2 * sizeof(ShotDev) + 33 * sizeof(float);
-  // at most 512 threads per SM for Born's two fields (128 registers a
-  // thread), 1024 for one
-  static constexpr int CAP = (BORN ? 512 : 1024) / G::NT;
+  // at most 512 threads per SM for Born's two fields and for the adjoint's
+  // imaging (128 registers a thread), 1024 for one field
+  static constexpr int CAP = (BORN || MODE == MODE_ADJ ? 512 : 1024) / G::NT;
   static constexpr int MIN_CTAS =
       ctas_fit(bytes + static_bytes, CAP) > 0 ? ctas_fit(bytes + static_bytes, CAP) : 1;
   static_assert((NCUR * CW * RW * sizeof(float)) % 128 == 0 && (TILE * sizeof(float)) % 128 == 0 &&
@@ -1315,7 +1359,7 @@ __global__ void __launch_bounds__(Geo<S>::NT, LCfg<S, MODE>::MIN_CTAS) interior_
   using ST = SAT<TZ>;  // the other arrays, the tile alone
   extern __shared__ __align__(128) unsigned char smraw[];
   float *stage0 = reinterpret_cast<float *>(smraw);
-  uint64_t *bar = reinterpret_cast<uint64_t *>(stage0 + 2 * L::STAGE);
+  uint64_t *bar = reinterpret_cast<uint64_t *>(stage0 + 2 * L::STAGE + L::WGT);
   __shared__ ShotDev sg[2];
   __shared__ int2 sxz[2];  // tile origin of each stage
   __shared__ float red[33];
@@ -1342,6 +1386,8 @@ __global__ void __launch_bounds__(Geo<S>::NT, LCfg<S, MODE>::MIN_CTAS) interior_
     int cur[2], oth[4];
     if (MODE == MODE_RCV) {
       cur[0] = MAP_FB_HALO + rcb; oth[0] = MAP_FB_TILE + rb; oth[1] = MAP_VEL_TILE;
+    } else if (L::ADJ) {
+      cur[0] = MAP_FA_HALO + rca; cur[1] = MAP_VEL_HALO; oth[0] = MAP_FA_TILE + ra;
     } else if (!BORN) {
       cur[0] = MAP_FA_HALO + rca; oth[0] = MAP_FA_TILE + ra; oth[1] = MAP_VEL_TILE;
     } else {
@@ -1379,19 +1425,24 @@ __global__ void __launch_bounds__(Geo<S>::NT, LCfg<S, MODE>::MIN_CTAS) interior_
     const ShotDev &g = sg[st];
     const int x0 = sxz[st].x, z0 = sxz[st].y;
     const int gzq[2] = {g.gz[x0 + cxq - g.pml] + g.pml, g.gz[x0 + cxq + 1 - g.pml] + g.pml};
+    Imager im;
+    if (L::ADJ) im.template load<TX, TZ>(g, a, x0, z0, x0 + cxq, z0 + 4 * (tid % QZ));
     // a wait that gives up leaves garbage in the stage (indices stay in
     // range); the CTA then ends after this tile
     if (!mbar_wait(bar + st, (par >> st) & 1u)) s_fail = 1;
     par ^= 1u << st;
-    const float *bb = stage0 + st * L::STAGE;
-    const float *ob = bb + L::NCUR * CW * RW;
-    const SW CA{bb, x0 - HI, z0 - HI};
-    const SW CB{bb + (BORN ? CW * RW : 0), x0 - HI, z0 - HI};
+    float *bb = stage0 + st * L::STAGE, *ob = bb + L::NCUR * CW * RW;
     const ST PA{ob, x0, z0};
-    const ST VV{ob + TILE, x0, z0};
-    const ST PB{ob + (BORN ? 2 : 0) * TILE, x0, z0};
-    const ST DV{ob + (BORN ? 3 : 1) * TILE, x0, z0};
-    interior_cells<S, MODE>(g, a, x0, z0, CA, CB, PA, PB, VV, DV, gzq, red);
+    if constexpr (L::ADJ) {
+      adj_interior_cells<S>(g, a, x0, z0, bb, bb + CW * RW, stage0 + 2 * L::STAGE, PA, gzq, im);
+    } else {
+      const SW CA{bb, x0 - HI, z0 - HI};
+      const SW CB{bb + (BORN ? CW * RW : 0), x0 - HI, z0 - HI};
+      const ST VV{ob + TILE, x0, z0};
+      const ST PB{ob + (BORN ? 2 : 0) * TILE, x0, z0};
+      const ST DV{ob + (BORN ? 3 : 1) * TILE, x0, z0};
+      interior_cells<S, MODE>(g, a, x0, z0, CA, CB, PA, PB, VV, DV, gzq, red);
+    }
     __syncthreads();  // stage st, its origin and shot table are free for the tile after next
     if (s_fail) {
       // the copies in flight into the other stage land before the CTA ends
