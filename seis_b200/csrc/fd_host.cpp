@@ -151,7 +151,8 @@ struct Plan {
   ShotDev *d_sd = nullptr;
   Tile *d_tiles = nullptr;
   int2 *d_cols = nullptr;
-  float *d_taps = nullptr;
+  float *d_taps = nullptr;  // adjointUpDown
+  HilbertTaps taps;         // the other imaging operators
   float *d_stage = nullptr;  // staging for unpadded uploads / transposes
   size_t stage_elems = 0;
   int NT = 0, nt = 0, ndel = 0, max_strip = 0, max_NZ = 0, max_tab = 0;
@@ -529,10 +530,9 @@ int plan_create(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *descs
     if (e == cudaSuccess && imaging) {
       e = cudaMemcpyAsync(p->d_cols, p->cols.data(), sizeof(int2) * p->cols.size(),
                           cudaMemcpyHostToDevice, st);
-      float taps[61];
-      hilbert_taps(taps, 30);
+      hilbert_taps(p->taps.h, 30);
       if (e == cudaSuccess)
-        e = cudaMemcpyAsync(p->d_taps, taps, sizeof taps, cudaMemcpyHostToDevice, st);
+        e = cudaMemcpyAsync(p->d_taps, p->taps.h, sizeof p->taps.h, cudaMemcpyHostToDevice, st);
       if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -731,23 +731,28 @@ int run_rtm_reverse(Plan &p) {
   }
   StepArgs a{};
   a.nshots = p.nshot;
-  a.src_k = -1;
-  a.strip_k = -1;
+  a.maps = p.d_maps;
+  // the imaging kernel also prepares the next step, where the boundary layers
+  // of a model do not meet
+  bool chain = true;
+  for (const ShotDev &g : p.sd) chain = chain && std::min(g.nx, g.nz) >= 2 * LAYERS;
   int k = 0;
   for (int it = p.NT - 1; it >= p.ndel; it--, k++) {
+    const bool first = it == p.NT - 1 || !chain;
+    if (first) {
+      CK(launch_rtm_restore(p.d_sd, p.nshot, p.max_strip, k, it, ctx->stream));
+      ctx->launches++;
+    }
     a.rot = k;
     a.rot_b = k;
-    CK(launch_rtm_restore(p.d_sd, p.nshot, p.max_strip, a.rot, it, ctx->stream));
-    ctx->launches++;
-    a.rec_k = -1;
-    int rc = step(p, MODE_MODEL, a);
-    if (rc) return rc;
     a.rec_k = it - p.ndel;
-    rc = step(p, MODE_RCV, a);
-    if (rc) return rc;
-    CK(launch_rtm_image(p.d_sd, p.d_cols, (int)p.cols.size(), a.rot, a.rot_b, p.max_NZ,
-                        p.d_taps, ctx->stream, p.op == OP_RTM_TRUE ? 2 : 0));
-    ctx->launches++;
+    a.pdl = !first;
+    CK(launch_pair(p.exact, p.d_sd, p.d_tiles, p.n_int, p.n_pad, p.shape, a, ctx->d_err,
+                   ctx->stream));
+    CK(launch_rtm_image(p.d_sd, p.d_cols, (int)p.cols.size(), a.rot, a.rot_b, p.max_NZ, p.taps,
+                        ctx->stream, p.op == OP_RTM_TRUE ? 2 : 0,
+                        chain && it > p.ndel ? it - 1 : -1, 1));
+    ctx->launches += 2;
   }
   return SEIS_OK;
 }
@@ -802,7 +807,7 @@ int run_rtm_plane(Plan &p) {
     rc = step(p, MODE_RCV, ra);
     if (rc) return rc;
     if (it - ndel > 0) {
-      CK(launch_rtm_image(p.d_sd, p.d_cols, (int)p.cols.size(), k, r0 + k, p.max_NZ, p.d_taps,
+      CK(launch_rtm_image(p.d_sd, p.d_cols, (int)p.cols.size(), k, r0 + k, p.max_NZ, p.taps,
                           ctx->stream, 1));
       ctx->launches++;
     }

@@ -234,7 +234,13 @@ cudaError_t launch_step(int mode, bool exact, const ShotDev *d_shots, const Tile
 // Whether such a step is two launches (the persistent interior kernel and the
 // pad tiles), or one of all tiles.
 bool step_splits(int mode, bool exact, int n_int, int shape, int loop);
+// One launch of a reverse step of the reference RTM: MODE_MODEL on field A and
+// MODE_RCV on field B (a.rot, a.rot_b, a.rec_k of the receivers).
+cudaError_t launch_pair(bool exact, const ShotDev *d_shots, const Tile *d_tiles, int n_int,
+                        int n_pad, int shape, const StepArgs &a, int *d_err, cudaStream_t s);
 namespace exact {
+cudaError_t launch_pair(const ShotDev *d_shots, const Tile *d_tiles, int n_int, int n_pad,
+                        int shape, const StepArgs &a, int *d_err, cudaStream_t s);
 cudaError_t launch_pad_tab(const ShotDev *d_shots, int nshots, int max_len, int born,
                            cudaStream_t s);
 bool step_splits(int mode, int n_int, int shape, int loop);
@@ -244,6 +250,8 @@ cudaError_t launch_step(int mode, const ShotDev *d_shots, const Tile *d_tiles, i
 cudaError_t configure();
 }  // namespace exact
 namespace fast {
+cudaError_t launch_pair(const ShotDev *d_shots, const Tile *d_tiles, int n_int, int n_pad,
+                        int shape, const StepArgs &a, int *d_err, cudaStream_t s);
 cudaError_t launch_pad_tab(const ShotDev *d_shots, int nshots, int max_len, int born,
                            cudaStream_t s);
 bool step_splits(int mode, int n_int, int shape, int loop);
@@ -286,9 +294,17 @@ cudaError_t launch_transpose(const float *d_src, int rows, int cols, float *d_ds
                              cudaStream_t s);
 cudaError_t launch_rtm_restore(const ShotDev *d_shots, int nshots, int max_strip, int rot,
                                int it, cudaStream_t s);
+// The 61-tap Hilbert filter of the imaging condition; taps passed by value (the
+// kernels read them from constant memory).
+struct HilbertTaps {
+  float h[61];
+};
+// restore_it >= 0: the kernel also prepares the next reverse step, of time step
+// restore_it, as launch_rtm_restore would (every model at least 8 x 8); pdl as
+// StepArgs::pdl.
 cudaError_t launch_rtm_image(const ShotDev *d_shots, const int2 *d_cols, int ncols, int rot,
-                             int rot_b, int max_nz, const float *d_taps, cudaStream_t s,
-                             int mode = 0);
+                             int rot_b, int max_nz, const HilbertTaps &taps, cudaStream_t s,
+                             int mode = 0, int restore_it = -1, int pdl = 0);
 cudaError_t launch_updown_image(const ShotDev *d_shots, const ShotDev *d_shots_h,
                                 const int2 *d_cols, int ncols, int rot, int rot_b, int max_nz,
                                 const float *d_taps, cudaStream_t s);

@@ -122,54 +122,129 @@ __global__ void plane_rcv_prep_kernel(const ShotDev *__restrict__ shots, int nsh
   cur[(size_t)ix * g.LDZ + iz] = src[i];  // SaveAtBoundary restore, fd.cpp:1206-1223
 }
 
+// Packed pairs (see V4 of the step kernels): a product rounded by itself is
+// x y + (-0), the zero read from constant memory.
+__constant__ float IMG_NEG_ZERO = -0.0f;
+__device__ __forceinline__ uint64_t bits2(const float2 &x) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x.x), "f"(x.y));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t x, uint64_t y, uint64_t nz) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(nz));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t x, uint64_t y) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+  return r;
+}
+__device__ __forceinline__ float2 pair2(uint64_t r) {
+  float2 x;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x.x), "=f"(x.y) : "l"(r));
+  return x;
+}
+
 // Imaging of the reference RTM, one CTA per interior column (fd.cpp:668-669,
 // :681-684, FaQi :1272-1298):
 //   U = ((u2 + u0 - 2 u1)/dt^2) vel3,  img += U R,  img += 0.5 (U R - H[U] H[R])
-// with H the 61-tap Hilbert FIR along z over the whole padded column.
+// with H the 61-tap Hilbert FIR along z over the whole padded column, whose
+// taps at even offsets are exactly zero (hilbert.h:67).  Bound by the filter's
+// arithmetic (30 products and sums of two fields, each rounded, per cell): U
+// and R lie interleaved in shared memory with HILB_HALF zeros on either side,
+// a thread forms IMG_K outputs two rows apart, so that each pair it reads
+// serves all of them and both fields share one packed operation; every third
+// pair of rows puts the 16 lanes of a half warp on different banks.  A column
+// of 320 rows: 210 -> 75 instructions a cell.
+// Then, when restore_it >= 0, the column's part of rtm_restore_kernel for the
+// next reverse step: nothing else reads these cells before it.
 constexpr int HILB_HALF = 30;
+constexpr int IMG_K = 3, IMG_THREADS = 128;
 // imaging of adjoint (lap vel3 R + FaQi), adjointPlane (FaQi of lap vel3),
 // rtm_true (FaQi of the source field times vel3)
 enum ImageMode { IMG_RTM = 0, IMG_PLANE = 1, IMG_TRUE = 2 };
-__global__ void rtm_image_kernel(const ShotDev *__restrict__ shots, const int2 *__restrict__ cols,
-                                 int rot, int rot_b, const float *__restrict__ taps, int mode) {
-  extern __shared__ float sh[];
+__global__ void __launch_bounds__(IMG_THREADS) rtm_image_kernel(
+    const ShotDev *__restrict__ shots, const int2 *__restrict__ cols, int rot, int rot_b,
+    const __grid_constant__ HilbertTaps taps, int mode, int restore_it) {
+  extern __shared__ float2 sUR[];  // HILB_HALF zeros, the column, zeros
   const int2 c = cols[blockIdx.x];
   const ShotDev &g = shots[c.x];
   const int ix = c.y + g.pml, NZ = g.NZ;
-  float *sU = sh, *sR = sh + NZ;
-  __shared__ float h[2 * HILB_HALF + 1];
-  if (threadIdx.x < 2 * HILB_HALF + 1) h[threadIdx.x] = taps[threadIdx.x];
   // reverse-pass naming: u2 = older (prev), u1 = current, u0 = newest
-  const float *u2 = g.fa[rot % 3], *u1 = g.fa[(rot + 1) % 3], *u0 = g.fa[(rot + 2) % 3];
-  const float *r0 = g.fb[(rot_b + 2) % 3];
   const size_t col = (size_t)ix * g.LDZ;
-  for (int iz = threadIdx.x; iz < NZ; iz += blockDim.x) {
-    float v = g.vel[col + iz];
-    float vel3 = 2.0f / (v * v * v);
+  const float *u2 = g.fa[rot % 3] + col, *r0 = g.fb[(rot_b + 2) % 3] + col;
+  float *u1 = g.fa[(rot + 1) % 3] + col, *u0 = g.fa[(rot + 2) % 3] + col;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  for (int i = threadIdx.x; i < HILB_HALF; i += IMG_THREADS)
+    sUR[i] = make_float2(0.0f, 0.0f);
+  // up to a whole group of outputs past the last row
+  for (int i = HILB_HALF + NZ + threadIdx.x; i < NZ + 2 * HILB_HALF + 2 * IMG_K; i += IMG_THREADS)
+    sUR[i] = make_float2(0.0f, 0.0f);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  for (int iz = threadIdx.x; iz < NZ; iz += IMG_THREADS) {
+    const float v = g.vel[col + iz];
+    const float vel3 = 2.0f / (v * v * v);
+    float u;
     if (mode == IMG_TRUE) {  // rtm_true images the source field itself, fd.cpp:1014
-      sU[iz] = u0[col + iz] * vel3;
+      u = u0[iz] * vel3;
     } else {
-      float lap = (u2[col + iz] + u0[col + iz] - 2.0f * u1[col + iz]) * g.idt2;
-      sU[iz] = lap * vel3;
+      const float lap = (u2[iz] + u0[iz] - 2.0f * u1[iz]) * g.idt2;
+      u = lap * vel3;
     }
-    sR[iz] = r0[col + iz];
+    sUR[HILB_HALF + iz] = make_float2(u, r0[iz]);
   }
   __syncthreads();
-  for (int iz = g.pml + threadIdx.x; iz < NZ - g.pml; iz += blockDim.x) {
-    int i0 = max(iz - HILB_HALF, 0), i1 = min(iz + HILB_HALF, NZ - 1);
-    float uh = 0.0f, rh = 0.0f;
-    // odd offsets only: the even taps are exactly zero (hilbert.h:67)
-    int start = i0 + (((iz - i0) & 1) ? 0 : 1);
-    for (int i = start; i <= i1; i += 2) {
-      float hk = h[iz - i + HILB_HALF];
-      uh = uh + sU[i] * hk;
-      rh = rh + sR[i] * hk;
+  const uint64_t nz = bits2(make_float2(IMG_NEG_ZERO, IMG_NEG_ZERO));
+  for (int q = threadIdx.x; 2 * IMG_K * (q >> 1) + (q & 1) < g.nz; q += IMG_THREADS) {
+    const int z0 = 2 * IMG_K * (q >> 1) + (q & 1);  // outputs z0, z0 + 2, ... (model rows)
+    const float2 *w = sUR + z0 + g.pml + 1;          // input z0 + pml - 29
+    uint64_t acc[IMG_K];
+#pragma unroll
+    for (int k = 0; k < IMG_K; k++) acc[k] = 0;
+    // input m (row z0 + pml - 29 + 2 m) meets output k at offset 2 (m - k) - 29,
+    // tap h[30 - offset]; each output sums by increasing row
+#pragma unroll
+    for (int m = 0; m < HILB_HALF + IMG_K - 1; m++) {
+      const uint64_t x = bits2(w[2 * m]);
+#pragma unroll
+      for (int k = 0; k < IMG_K; k++) {
+        const int n = m - k;
+        if (n < 0 || n >= HILB_HALF) continue;
+        const float h = taps.h[HILB_HALF - (2 * n - 29)];
+        acc[k] = add2(acc[k], mul2(x, bits2(make_float2(h, h)), nz));
+      }
     }
-    float U = sU[iz], R = sR[iz];
-    float *img = g.img + (size_t)c.y * g.nz + (iz - g.pml);
-    float acc = mode == IMG_RTM ? *img + U * R : *img;  // the others image with FaQi alone
-    acc = acc + 0.5f * (U * R - uh * rh);
-    *img = acc;
+#pragma unroll
+    for (int k = 0; k < IMG_K; k++) {
+      const int z = z0 + 2 * k;
+      if (z >= g.nz) break;
+      const float2 ur = sUR[HILB_HALF + g.pml + z], f = pair2(acc[k]);
+      float *img = g.img + (size_t)c.y * g.nz + z;
+      float a = mode == IMG_RTM ? *img + ur.x * ur.y : *img;  // the others image with FaQi alone
+      a = a + 0.5f * (ur.x * ur.y - f.x * f.y);
+      *img = a;
+    }
+  }
+  if (restore_it < 0 || restore_it >= g.NT || restore_it < g.ndel) return;
+  __syncthreads();  // the column's fields have been read
+  // the source off the field that is the older one of the next step (a source
+  // outside the model's columns: the first column's CTA, as no other reads it)
+  const bool mine = ix == g.sxp || (c.y == 0 && (g.sxp < g.pml || g.sxp >= g.pml + g.nx));
+  if (threadIdx.x == 0 && restore_it - 1 > 0 && mine) {
+    const size_t off = (size_t)g.sxp * g.LDZ + g.szp;
+    float *prev = g.fa[(rot + 1) % 3];
+    prev[off] = prev[off] - coef(g.vel[off], g).vt2 * g.wav[restore_it - 1];
+  }
+  // the saved boundary layers of the sample into the newest field
+  const float *src = g.strips + (size_t)(restore_it - g.ndel) * g.strip_len;
+  const int edge = c.y < LAYERS ? c.y : c.y >= g.nx - LAYERS ? LAYERS + (g.nx - 1 - c.y) : -1;
+  if (edge >= 0) {
+    const float *s = src + 2 * LAYERS * g.nx + edge * g.nz;
+    for (int z = threadIdx.x; z < g.nz; z += IMG_THREADS) u0[g.pml + z] = s[z];
+  } else if (threadIdx.x < 2 * LAYERS) {
+    const int l = threadIdx.x;
+    u0[l < LAYERS ? g.pml + l : g.nz + g.pml - 1 - (l - LAYERS)] = src[l * g.nx + c.y];
   }
 }
 
@@ -263,6 +338,12 @@ cudaError_t launch_step(int mode, bool use_exact, const ShotDev *d_shots, const 
                                        s_int, s_pad);
 }
 
+cudaError_t launch_pair(bool use_exact, const ShotDev *d_shots, const Tile *d_tiles, int n_int,
+                        int n_pad, int shape, const StepArgs &a, int *d_err, cudaStream_t s) {
+  return use_exact ? exact::launch_pair(d_shots, d_tiles, n_int, n_pad, shape, a, d_err, s)
+                   : fast::launch_pair(d_shots, d_tiles, n_int, n_pad, shape, a, d_err, s);
+}
+
 bool step_splits(int mode, bool use_exact, int n_int, int shape, int loop) {
   return use_exact ? exact::step_splits(mode, n_int, shape, loop)
                    : fast::step_splits(mode, n_int, shape, loop);
@@ -297,16 +378,26 @@ cudaError_t launch_rtm_restore(const ShotDev *d_shots, int nshots, int max_strip
 }
 
 cudaError_t launch_rtm_image(const ShotDev *d_shots, const int2 *d_cols, int ncols, int rot,
-                             int rot_b, int max_nz, const float *d_taps, cudaStream_t s,
-                             int mode) {
-  size_t smem = 2 * (size_t)max_nz * sizeof(float);
+                             int rot_b, int max_nz, const HilbertTaps &taps, cudaStream_t s,
+                             int mode, int restore_it, int pdl) {
+  const size_t smem = ((size_t)max_nz + 2 * HILB_HALF + 2 * IMG_K) * sizeof(float2);
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(rtm_image_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  rtm_image_kernel<<<ncols, 256, smem, s>>>(d_shots, d_cols, rot, rot_b, d_taps, mode);
-  return cudaGetLastError();
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(ncols);
+  c.blockDim = dim3(IMG_THREADS);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&c, rtm_image_kernel, d_shots, d_cols, rot, rot_b, taps, mode,
+                            restore_it);
 }
 
 cudaError_t launch_updown_image(const ShotDev *d_shots, const ShotDev *d_shots_h,

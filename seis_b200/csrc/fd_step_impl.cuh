@@ -118,7 +118,27 @@ cudaError_t setup_shape() {
 #ifdef SEIS_FAST_MATH
   if (e == cudaSuccess) e = setup<S, MODE_ADJ>();
 #endif
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(step_pair_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)UCfg<S, MODE_MODEL>::bytes);
   return e;
+}
+
+// A launch that may start before the last one on the stream has finished
+// (programmatic) when `pdl`.
+template <class K, class... A>
+cudaError_t launch_pdl(K kernel, int grid, int block, size_t smem, cudaStream_t s, int pdl, A... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kernel, args...);
 }
 
 // Every tile in one launch on s_int, or the interior tiles by the persistent
@@ -144,18 +164,9 @@ cudaError_t launch_t(const ShotDev *d_shots, const Tile *d_tiles, int n_int, int
     n_int = 0;
   }
   if (n_int + n_pad > 0) {
-    cudaLaunchConfig_t c = {};
-    c.gridDim = dim3(n_int + n_pad);
-    c.blockDim = dim3(NT);
-    c.dynamicSmemBytes = UCfg<S, MODE>::bytes;
-    c.stream = n_int > 0 ? s_int : s_pad;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = at;
-    c.numAttrs = a.pdl ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&c, step_tile_kernel<S, MODE>, d_shots, d_tiles, n_int,
-                                       n_pad, a, d_err);
+    cudaError_t e = launch_pdl(step_tile_kernel<S, MODE>, n_int + n_pad, NT, UCfg<S, MODE>::bytes,
+                               n_int > 0 ? s_int : s_pad, a.pdl, d_shots, d_tiles, n_int, n_pad, a,
+                               d_err);
     if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
@@ -215,6 +226,24 @@ cudaError_t configure() {
   if (e == cudaSuccess) e = setup_shape<SHAPE_64x64>();
   if (e == cudaSuccess) e = setup_shape<SHAPE_32x32>();
   return e;
+}
+
+template <int S>
+static cudaError_t launch_pair_s(const ShotDev *d_shots, const Tile *d_tiles, int n_int, int n_pad,
+                                 const StepArgs &a, int *d_err, cudaStream_t s) {
+  return launch_pdl(step_pair_kernel<S>, 2 * (n_int + n_pad), Geo<S>::NT,
+                    UCfg<S, MODE_MODEL>::bytes, s, a.pdl, d_shots, d_tiles, n_int, n_pad, a, d_err);
+}
+cudaError_t launch_pair(const ShotDev *d_shots, const Tile *d_tiles, int n_int, int n_pad,
+                        int shape, const StepArgs &a, int *d_err, cudaStream_t s) {
+  switch (shape) {
+    case SHAPE_32x64: return launch_pair_s<SHAPE_32x64>(d_shots, d_tiles, n_int, n_pad, a, d_err, s);
+    case SHAPE_64x32: return launch_pair_s<SHAPE_64x32>(d_shots, d_tiles, n_int, n_pad, a, d_err, s);
+    case SHAPE_16x128: return launch_pair_s<SHAPE_16x128>(d_shots, d_tiles, n_int, n_pad, a, d_err, s);
+    case SHAPE_64x64: return launch_pair_s<SHAPE_64x64>(d_shots, d_tiles, n_int, n_pad, a, d_err, s);
+    case SHAPE_32x32: return launch_pair_s<SHAPE_32x32>(d_shots, d_tiles, n_int, n_pad, a, d_err, s);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 cudaError_t launch_step(int mode, const ShotDev *d_shots, const Tile *d_tiles, int n_int,

@@ -1211,9 +1211,8 @@ __device__ __forceinline__ bool pad_cells(const ShotDev &g, const StepArgs &a, i
 // shots in the exact build 57 -> 28 us (16 B per cell at the copy rate: 12 us);
 // the pad tiles of eight Born shots of 4000 x 1000: 84 -> 68 us.
 template <int S, int MODE>
-__global__ void __launch_bounds__(Geo<S>::NT, UCfg<S, MODE>::MIN_CTAS) step_tile_kernel(
-    const ShotDev *__restrict__ shots, const Tile *__restrict__ tiles, int n_int, int n_pad,
-    StepArgs a, int *__restrict__ err) {
+__device__ __forceinline__ void tile_step(const ShotDev *__restrict__ shots, const Tile &t,
+                                          const StepArgs &a, int *__restrict__ err) {
   SEIS_GEO(S);
   using K = UCfg<S, MODE>;
   constexpr bool BORN = K::BORN;
@@ -1224,7 +1223,6 @@ __global__ void __launch_bounds__(Geo<S>::NT, UCfg<S, MODE>::MIN_CTAS) step_tile
   __shared__ ShotDev sg;
   __shared__ float red[33];
   const int tid = threadIdx.x;
-  const Tile t = tiles[(int)blockIdx.x < n_pad ? n_int + (int)blockIdx.x : (int)blockIdx.x - n_pad];
   const bool pad = t.kind == TILE_PAD;
   pdl_trigger();
   if (tid == NT_T - 32) {  // the last warp's first lane, while the others fetch the shot table
@@ -1314,6 +1312,35 @@ __global__ void __launch_bounds__(Geo<S>::NT, UCfg<S, MODE>::MIN_CTAS) step_tile
       const ST V{sm + K::O_V, t.x0, t.z0}, D{sm + K::O_D, t.x0, t.z0};
       interior_cells<S, MODE>(g, a, t.x0, t.z0, CA, CB, PA, PB, V, D, gzq, red);
     }
+  }
+}
+
+template <int S, int MODE>
+__global__ void __launch_bounds__(Geo<S>::NT, UCfg<S, MODE>::MIN_CTAS) step_tile_kernel(
+    const ShotDev *__restrict__ shots, const Tile *__restrict__ tiles, int n_int, int n_pad,
+    StepArgs a, int *__restrict__ err) {
+  const int b = blockIdx.x;
+  tile_step<S, MODE>(shots, tiles[b < n_pad ? n_int + b : b - n_pad], a, err);
+}
+
+// One reverse step of the reference RTM: the source field (A) reconstructed
+// and the receiver field (B) propagated, which do not depend on one another,
+// in one launch over the tile list twice (the pad tiles of both first).  As
+// two launches on single shots each waited for the other's last tile.
+template <int S>
+__global__ void __launch_bounds__(Geo<S>::NT, UCfg<S, MODE_MODEL>::MIN_CTAS) step_pair_kernel(
+    const ShotDev *__restrict__ shots, const Tile *__restrict__ tiles, int n_int, int n_pad,
+    StepArgs a, int *__restrict__ err) {
+  static_assert(UCfg<S, MODE_MODEL>::bytes == UCfg<S, MODE_RCV>::bytes, "one launch for both");
+  int b = blockIdx.x;
+  const bool rcv = b & 1;
+  b >>= 1;
+  const Tile t = tiles[b < n_pad ? n_int + b : b - n_pad];
+  if (rcv) {
+    tile_step<S, MODE_RCV>(shots, t, a, err);
+  } else {
+    a.rec_k = -1;
+    tile_step<S, MODE_MODEL>(shots, t, a, err);
   }
 }
 
