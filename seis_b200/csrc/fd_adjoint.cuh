@@ -322,25 +322,43 @@ __device__ __noinline__ float4 ring_cell(const ShotDev &g, const AdjTab<TX, TZ> 
   return make_float4(m, e, b, 0.0f);
 }
 
-// The terms are summed in ring_cell's order: by column, rows fastest.
+// Where one target quad (column cx, rows iz0 .. iz0+3) sits: kind 0, every
+// ring cell around it lies in one top or bottom strip; 1, in one left or right
+// strip; 2, anything else.
+struct RingQuad {
+  int Dl, Dc, Dr, kind;
+  bool upper, left;
+  __device__ __forceinline__ RingQuad(const ShotDev &g, int cx, int iz0) {
+    Dl = dist_x(g, cx - 1), Dc = dist_x(g, cx), Dr = dist_x(g, cx + 1);
+    const int Za = dist_z(g, iz0 - 1), Zb = dist_z(g, iz0 + 4);
+    const int Dmax = max(max(Dl, Dr), Dc), Dmin = min(min(Dl, Dr), Dc);
+    const bool lower = iz0 + 4 >= g.pml + g.nz, right = cx + 1 >= g.pml + g.nx;
+    upper = iz0 - 1 < g.pml;
+    left = cx - 1 < g.pml;
+    // largest and smallest distance along z over the rows iz0 - 1 .. iz0 + 4
+    const bool twice = upper && lower;
+    const int Zmax = max(Za, Zb), Zmin = twice ? 0 : min(Za, Zb);
+    kind = !twice && (Dmax == 0 || Zmin > Dmax) ? 0
+           : !(left && right) && (Zmax == 0 || (Dmin > Zmax && !twice)) ? 1 : 2;
+  }
+};
+
+// The terms of a quad of kind 0 or 1, summed in ring_cell's order: by column,
+// rows fastest.
 template <int TX, int TZ, class UA_>
-__device__ __forceinline__ RingTerms ring_quad(const ShotDev &g, const AdjTab<TX, TZ> &T,
-                                               const UA_ &U, int x0, int z0, int cx, int iz0) {
+__device__ __forceinline__ RingTerms ring_quad(const ShotDev &g, const RingQuad &k,
+                                               const AdjTab<TX, TZ> &T, const UA_ &U, int x0,
+                                               int z0, int cx, int iz0) {
   RingTerms o;
-  const int Dl = dist_x(g, cx - 1), Dc = dist_x(g, cx), Dr = dist_x(g, cx + 1);
-  const int Za = dist_z(g, iz0 - 1), Zb = dist_z(g, iz0 + 4);
-  const int Dmax = max(max(Dl, Dr), Dc), Dmin = min(min(Dl, Dr), Dc);
-  const bool upper = iz0 - 1 < g.pml, lower = iz0 + 4 >= g.pml + g.nz;
-  const bool left = cx - 1 < g.pml, right = cx + 1 >= g.pml + g.nx;
-  // largest and smallest distance along z over the rows iz0 - 1 .. iz0 + 4
-  const int Zmax = max(Za, Zb), Zmin = upper && lower ? 0 : min(Za, Zb);
+  const int Dl = k.Dl, Dc = k.Dc, Dr = k.Dr;
+  const bool upper = k.upper, left = k.left;
   const V4 one = v4(1.0f);
   auto weight = [&](const V4 &d) { return fma4(d, v4(-g.inv_pml), one); };
   const V4 Zq = dist_quad(g, iz0);
   const float4 q = U.quad(cx, iz0);
   o.w = weight(Dc > 0 ? v4((float)Dc) : Zq);
   // every ring cell around the quad in one top or bottom strip
-  if (!(upper && lower) && (Dmax == 0 || Zmin > Dmax)) {
+  if (k.kind == 0) {
     const float(*t)[AdjTab<TX, TZ>::NC] = T.z[!upper];
     const int c = cx - x0 + ADJ_TAB_M;
     const float al = t[0][c], bl = t[1][c - 1], br = t[1][c + 1], ga = t[2][c];
@@ -375,7 +393,7 @@ __device__ __forceinline__ RingTerms ring_quad(const ShotDev &g, const AdjTab<TX
     return o;
   }
   // in one left or right strip
-  if (!(left && right) && (Zmax == 0 || Dmin > Zmax) && !(upper && lower && Zmax > 0)) {
+  {
     const float(*t)[AdjTab<TX, TZ>::NR] = T.x[!left];
     const int r = iz0 - z0 + ADJ_TAB_M, xn = left ? cx - 1 : cx + 1;
     const V4 wn = one - weight(v4((float)(left ? Dl : Dr))), wc = one - weight(v4((float)Dc));
@@ -398,19 +416,6 @@ __device__ __forceinline__ RingTerms ring_quad(const ShotDev &g, const AdjTab<TX
     }
     return o;
   }
-  float m[4], e[4], b[4];
-#pragma unroll 1
-  for (int r = 0; r < 4; r++) {
-    const float4 t = ring_cell<TX, TZ>(g, T, U, x0, z0, cx, iz0 + r);
-    if (r == 0) m[0] = t.x, e[0] = t.y, b[0] = t.z;
-    if (r == 1) m[1] = t.x, e[1] = t.y, b[1] = t.z;
-    if (r == 2) m[2] = t.x, e[2] = t.y, b[2] = t.z;
-    if (r == 3) m[3] = t.x, e[3] = t.y, b[3] = t.z;
-  }
-  o.m = v4(make_float4(m[0], m[1], m[2], m[3]));
-  o.e = v4(make_float4(e[0], e[1], e[2], e[3]));
-  o.b = v4(make_float4(b[0], b[1], b[2], b[3]));
-  return o;
 }
 
 // vx M1 over the staged velocity `v` and vz M1 into `wz` of a quad
@@ -479,7 +484,8 @@ __device__ __forceinline__ void adj_interior_cells(const ShotDev &g, const StepA
 template <int S>
 __device__ __forceinline__ bool adj_pad_cells(const ShotDev &g, const StepArgs &a, int x0, int z0,
                                               float *sm, uint64_t *tab_bar, const int (&gzq)[2],
-                                              const Imager &im) {
+                                              const QuadSort<Geo<S>::TX * Geo<S>::QZ> &sort,
+                                              bool corner, const Imager &im) {
   SEIS_GEO(S);
   using SA = SAT<SR>;
   using K = UCfg<S, MODE_ADJ>;
@@ -602,25 +608,43 @@ __device__ __forceinline__ bool adj_pad_cells(const ShotDev &g, const StepArgs &
   const QuadList aff(x0, z0, xe, ze, g.pml + 1, g.pml + g.nx - 1, g.pml + 1, g.pml + g.nz - 1);
   constexpr int KMAX = (TX * QZ + NT_T - 1) / NT_T;
   float4 bold[KMAX];
+  const int npure = corner ? sort.nz + sort.nx : aff.n;
+  auto quad_of = [&](int e, int &cx, int &dz) { aff.quad(corner ? sort.get(e) : e, cx, dz); };
 #pragma unroll
   for (int k = 0; k < KMAX; k++) {
-    const int i = tid + k * NT_T;
-    if (i < aff.n) {
+    const int e = tid + k * NT_T;
+    if (e < npure) {
       int cx, dz;
-      aff.quad(i, cx, dz);
+      quad_of(e, cx, dz);
       bold[k] = *reinterpret_cast<const float4 *>(g.adj_b + (size_t)cx * g.LDZ + z0 + dz);
     }
   }
   const bool landed = mbar_wait(tab_bar, 0);
   __syncthreads();
+  // one cell by the general gather
+  auto general = [&](int cx, int iz) {
+    const float4 t = ring_cell<TX, TZ>(g, tab, U, x0, z0, cx, iz);
+    const int D = dist_x(g, cx), Z = dist_z(g, iz);
+    const float w = __fmaf_rn(-(float)(D > 0 ? D : Z), g.inv_pml, 1.0f);
+    const size_t at = (size_t)cx * g.LDZ + iz;
+    out[at] = __fmaf_rn(w, U(cx, iz), t.x);
+    Enext[at] = t.y + g.adj_b[at];
+    g.adj_b[at] = t.z;
+  };
 #pragma unroll
   for (int k = 0; k < KMAX; k++) {
     const int i = tid + k * NT_T;
-    if (i >= aff.n) continue;
+    if (i >= npure) continue;
     int cx, dz;
-    aff.quad(i, cx, dz);
+    quad_of(i, cx, dz);
     const int iz = z0 + dz;
-    const RingTerms t = ring_quad<TX, TZ>(g, tab, U, x0, z0, cx, iz);
+    const RingQuad rq(g, cx, iz);
+    if (rq.kind == 2) {  // not in a corner tile: a model of a few cells
+#pragma unroll 1
+      for (int r = 0; r < 4 && iz + r < NZ; r++) general(cx, iz + r);
+      continue;
+    }
+    const RingTerms t = ring_quad<TX, TZ>(g, rq, tab, U, x0, z0, cx, iz);
     const size_t at = (size_t)cx * g.LDZ + iz;
     const float4 n = f4(fma4(t.w, v4(U.quad(cx, iz)), t.m));
     const float4 e = f4(t.e + v4(bold[k])), b = f4(t.b);
@@ -637,6 +661,13 @@ __device__ __forceinline__ bool adj_pad_cells(const ShotDev &g, const StepArgs &
           g.adj_b[at + r] = comp(b, r);
         }
     }
+  }
+  // the corner tile's other quads, a cell per thread
+  for (int j = tid; corner && j < 4 * sort.nm; j += NT_T) {
+    int cx, dz;
+    aff.quad(sort.mixed[j >> 2], cx, dz);
+    const int iz = z0 + dz + (j & 3);
+    if (iz < NZ) general(cx, iz);
   }
   return landed;
 }
