@@ -35,10 +35,12 @@ struct seis_fd_ctx {
   cudaStream_t stream = nullptr;  // all work is ordered on this stream
   cudaStream_t aux = nullptr;     // boundary tiles run here, joined every step
   cudaEvent_t fork = nullptr, join = nullptr;
-  int *d_err = nullptr;  // set by kernels whose bounded waits ran out
+  // host memory mapped into the device, which the host reads after waiting for
+  // the stream: a copy of a word to the host costs as much again as the wait
+  int *d_err = nullptr;        // set by kernels whose bounded waits ran out
   std::vector<seis_fd_plan *> plans;  // live plans, torn down with the context
   double *d_partial = nullptr;        // DOT_PARTS partial sums of a dot product
-  double *d_scalar = nullptr;         // one FP64 result
+  double *d_scalar = nullptr;         // one FP64 result (mapped, as d_err)
   int num_sms = 148;
   std::string err;
   int64_t launches = 0;
@@ -411,7 +413,8 @@ int make_hilbert_table(Plan &p) {
   return SEIS_OK;
 }
 
-int plan_create(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *descs, Plan **out) {
+int plan_create(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *descs, Plan **out,
+                int shape = SHAPE_32x64) {
   *out = nullptr;
   if (nshot < 1 || !descs) return fail(ctx, SEIS_ERR_ARG, "nshot=%d", nshot);
   for (int i = 0; i < nshot; i++) {
@@ -429,6 +432,7 @@ int plan_create(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *descs
   if (!p) return fail(ctx, SEIS_ERR_NOMEM, "host allocation failed");
   p->ctx = ctx;
   p->op = op;
+  p->shape = shape;
   p->nshot = nshot;
   p->desc.assign(descs, descs + nshot);
   p->gz.resize(nshot);
@@ -1074,10 +1078,9 @@ int download_gather(Plan &p, int s, float *h_rec) {
 
 int sync(seis_fd_ctx *ctx) {
   CK(cudaStreamSynchronize(ctx->stream));
-  int flag = 0;
-  CK(cudaMemcpy(&flag, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+  const int flag = *static_cast<volatile int *>(ctx->d_err);
   if (flag) {
-    CK(cudaMemset(ctx->d_err, 0, sizeof(int)));
+    *static_cast<volatile int *>(ctx->d_err) = 0;
     return fail(ctx, SEIS_ERR_CUDA, "a kernel gave up waiting for its staged input (code %d)", flag);
   }
   return SEIS_OK;
@@ -1138,10 +1141,11 @@ int seis_fd_create(seis_fd_ctx **out, int device) {
   if (e == cudaSuccess) e = configure_kernels();
   if (e == cudaSuccess)
     e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
-  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_err, sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_partial, sizeof(double) * DOT_PARTS);
-  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_scalar, sizeof(double));
-  if (e == cudaSuccess) e = cudaMemset(ctx->d_err, 0, sizeof(int));
+  if (e == cudaSuccess) e = cudaHostAlloc(&ctx->d_err, sizeof(int), cudaHostAllocMapped);
+  if (e == cudaSuccess) e = cudaHostAlloc(&ctx->d_scalar, sizeof(double), cudaHostAllocMapped);
+  if (e == cudaSuccess) *ctx->d_err = 0;
+  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_partial, sizeof(double) * (DOT_PARTS + 1));
+  if (e == cudaSuccess) e = cudaMemset(ctx->d_partial, 0, sizeof(double) * (DOT_PARTS + 1));
   if (e != cudaSuccess) {
     seis_fd_destroy(ctx);
     return SEIS_ERR_CUDA;
@@ -1163,9 +1167,9 @@ int seis_fd_destroy(seis_fd_ctx *ctx) {
   ctx->plans.clear();
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->aux) cudaStreamSynchronize(ctx->aux);
-  if (ctx->d_err) cudaFree(ctx->d_err);
+  if (ctx->d_err) cudaFreeHost(ctx->d_err);
   if (ctx->d_partial) cudaFree(ctx->d_partial);
-  if (ctx->d_scalar) cudaFree(ctx->d_scalar);
+  if (ctx->d_scalar) cudaFreeHost(ctx->d_scalar);
   if (ctx->fork) cudaEventDestroy(ctx->fork);
   if (ctx->join) cudaEventDestroy(ctx->join);
   if (ctx->aux) cudaStreamDestroy(ctx->aux);
@@ -1471,8 +1475,10 @@ int apply_shape(Plan &p, int s) {
 std::mutex g_tune_mu;
 std::map<std::string, int> g_tune_cache;
 
+bool fp16_scales(const Plan &p) { return p.op == OP_BORN_ADJ && p.snap_dtype == SNAP_F16; }
+
 std::string tune_key(const Plan &p) {
-  std::string k = std::to_string(p.op) + (p.exact ? "e" : "f");
+  std::string k = std::to_string(p.op) + (p.exact ? "e" : "f") + (fp16_scales(p) ? "h" : "");
   for (const ShotDev &g : p.sd) k += ":" + std::to_string(g.NX) + "x" + std::to_string(g.NZ);
   return k;
 }
@@ -1510,13 +1516,13 @@ int autotune(Plan &p, int steps, bool force, double *ms, int *best) {
       return apply(it->second);
     }
   }
-  // An adjoint plan's shape is also the tiling of its 16-bit snapshots' scales,
-  // so a choice within the noise of the timing would change its results in
-  // their last bits from one process to the next: it stays at 64x32, at or
-  // near the fastest from a few hundred to a few thousand tiles (lead of the
-  // best of the others: at most 5% over 25 surveys), unless another shape
-  // leads by 8%.
-  const bool steady = p.op == OP_BORN_ADJ;
+  // An adjoint plan's shape is also the tiling of its FP16 snapshots' scales,
+  // and small values lie in FP16's denormal range by their tile's scale: a
+  // choice by time would change its results in their last bits from one
+  // process to the next.  Such a plan stays at 64x32, the fastest shape of
+  // most surveys from a hundred to some thousand tiles and within 10% of the
+  // fastest in the others; its launch form is chosen by time.
+  const bool steady = fp16_scales(p);
   int pick = 0, pick_steady = 0;
   double t_best = 0.0, t_steady = 0.0;
   for (int c = 0; c < 4 * NSHAPES; c++) {
@@ -1536,7 +1542,7 @@ int autotune(Plan &p, int steps, bool force, double *ms, int *best) {
       pick_steady = c;
     }
   }
-  if (steady && t_steady < 1.08 * t_best) pick = pick_steady;
+  if (steady) pick = pick_steady;
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     g_tune_cache[key] = pick;
@@ -1641,7 +1647,12 @@ static int run_batch(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *
   if (!in1 || !in2 || (what3 >= 0 && !in3) || !out)
     return fail(ctx, SEIS_ERR_ARG, "null array list");
   Plan *p = nullptr;
-  rc = plan_create(ctx, op, nshot, shots, &p);
+  // one-field steps are fastest in 32x32 tiles (281 x 281: 8.7 us against 10.1 in
+  // 32x64; eight of 1280 x 480: 24.7 against 28.5), the adjoint's reverse step in 64x32
+  // (24.6 against 26.9 us), Born and RTM in 32x64 (15.0 against 15.7 us)
+  const int shape = op == OP_MODEL || op == OP_ILLUM || op == OP_ILLUM_PLANE ? SHAPE_32x32
+                    : op == OP_BORN_ADJ ? SHAPE_64x32 : SHAPE_32x64;
+  rc = plan_create(ctx, op, nshot, shots, &p, shape);
   if (rc) return rc;
   seis_fd_plan h{p};
   for (int s = 0; s < nshot && !rc; s++) {
@@ -1801,9 +1812,10 @@ int seis_fd_vec_dot(seis_fd_ctx *ctx, const float *d_a, const float *d_b, size_t
   if (rc) return rc;
   if (!d_a || !d_b || !h_out) return fail(ctx, SEIS_ERR_ARG, "null pointer");
   CK(launch_dot(d_a, d_b, n, ctx->d_partial, ctx->d_scalar, 0, ctx->stream));
-  ctx->launches += 2;
-  CK(cudaMemcpyAsync(h_out, ctx->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  return sync(ctx);
+  ctx->launches++;
+  rc = sync(ctx);
+  if (!rc) *h_out = *static_cast<volatile double *>(ctx->d_scalar);
+  return rc;
 }
 
 int seis_fd_vec_axpby(seis_fd_ctx *ctx, float *d_y, const float *d_x, double a, double b,
@@ -2015,7 +2027,7 @@ int data_dot(seis_fd_lsrtm &L, bool q_left, bool q_right, double *out) {
     const float *q = lsrtm_q(L, k), *r = L.r + L.doff[k];
     size_t n = (size_t)L.shots[k].nx * L.nt;
     CK(launch_dot(q_left ? q : r, q_right ? q : r, n, ctx->d_partial, out, k > 0, ctx->stream));
-    ctx->launches += 2;
+    ctx->launches++;
   }
   return SEIS_OK;
 }
@@ -2288,7 +2300,7 @@ int seis_fd_lsrtm_phase_direction(seis_fd_lsrtm *L, const float *d_s, int first)
   if (d_s != L->s)
     CK(cudaMemcpyAsync(L->s, d_s, sizeof(float) * nm, cudaMemcpyDeviceToDevice, ctx->stream));
   CK(launch_dot(L->s, L->s, nm, ctx->d_partial, gnew, 0, ctx->stream));
-  ctx->launches += 2;
+  ctx->launches++;
   if (first) {
     CK(cudaMemcpyAsync(gamma, gnew, sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
     CK(cudaMemcpyAsync(L->p, L->s, sizeof(float) * nm, cudaMemcpyDeviceToDevice, ctx->stream));

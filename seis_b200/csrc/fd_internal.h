@@ -273,7 +273,9 @@ cudaError_t launch_pad_tab(bool exact, const ShotDev *d_shots, int nshots, int m
 cudaError_t launch_finalize_image(const ShotDev *d_shots, int nshots, cudaStream_t s);
 
 // Vector operations of the CG solver (fd_vec.cu).  A dot product needs a
-// scratch array of DOT_PARTS doubles for its per-CTA partial sums.
+// scratch array of DOT_PARTS doubles for its per-CTA partial sums and one more
+// word, zero before its first use; launches that share it run one after the
+// other.  out: device memory, or host memory mapped into the device.
 constexpr int DOT_PARTS = 1184;
 cudaError_t launch_dot(const float *a, const float *b, size_t n, double *partial, double *out,
                        int accumulate, cudaStream_t s);
