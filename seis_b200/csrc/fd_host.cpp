@@ -150,6 +150,11 @@ struct Plan {
   int loop = -1;  // interior kernel form (StepArgs::loop)
   std::vector<void *> allocs;
   std::vector<size_t> alloc_bytes;
+  // one cleared allocation that alloc() carves the plan's arrays from (what
+  // does not fit is allocated by itself): with ten arrays a shot, allocating
+  // and freeing them one by one took 33 ms of a 47 ms call over 16 shots
+  unsigned char *slab = nullptr;
+  size_t slab_size = 0, slab_used = 0;
   ShotDev *d_sd = nullptr;
   Tile *d_tiles = nullptr;
   int2 *d_cols = nullptr;
@@ -166,13 +171,33 @@ struct Plan {
   ~Plan() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
-    for (void *p : allocs) cudaFree(p);
+    for (void *p : allocs)
+      if (!in_slab(p)) cudaFree(p);
+    if (slab) cudaFree(slab);
+  }
+  bool in_slab(const void *q) const {
+    const unsigned char *c = static_cast<const unsigned char *>(q);
+    return slab && c >= slab && c < slab + slab_size;
+  }
+  static size_t rounded(size_t bytes) { return (std::max<size_t>(bytes, 1) + 255) / 256 * 256; }
+  // the slab; without the memory for it in one piece the arrays are allocated
+  // one by one
+  int reserve(size_t bytes) {
+    if (cudaMalloc(&slab, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      slab = nullptr;
+      return SEIS_OK;
+    }
+    slab_size = bytes;
+    cudaError_t e = cudaMemsetAsync(slab, 0, bytes, ctx->stream);
+    return e == cudaSuccess ? SEIS_OK
+                            : fail(ctx, SEIS_ERR_CUDA, "cudaMemset: %s", cudaGetErrorString(e));
   }
   // free one allocation made by alloc() (null: nothing)
   void release(void *q) {
     for (size_t i = 0; q && i < allocs.size(); i++)
       if (allocs[i] == q) {
-        cudaFree(q);
+        if (!in_slab(q)) cudaFree(q);
         device_bytes -= (int64_t)alloc_bytes[i];
         allocs.erase(allocs.begin() + i);
         alloc_bytes.erase(alloc_bytes.begin() + i);
@@ -182,7 +207,15 @@ struct Plan {
   template <class T>
   int alloc(T **p, size_t n) {
     void *q = nullptr;
-    cudaError_t e = cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T));
+    const size_t room = rounded(n * sizeof(T));
+    const bool carve = slab && room <= slab_size - slab_used;
+    cudaError_t e = cudaSuccess;
+    if (carve) {
+      q = slab + slab_used;
+      slab_used += room;
+    } else {
+      e = cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T));
+    }
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(ctx, e == cudaErrorMemoryAllocation ? SEIS_ERR_NOMEM : SEIS_ERR_CUDA,
@@ -192,6 +225,7 @@ struct Plan {
     alloc_bytes.push_back(std::max<size_t>(n, 1) * sizeof(T));
     device_bytes += (int64_t)(std::max<size_t>(n, 1) * sizeof(T));
     *p = static_cast<T *>(q);
+    if (carve) return SEIS_OK;  // cleared with the slab
     e = cudaMemsetAsync(q, 0, std::max<size_t>(n, 1) * sizeof(T), ctx->stream);
     if (e != cudaSuccess) return fail(ctx, SEIS_ERR_CUDA, "cudaMemset: %s", cudaGetErrorString(e));
     return SEIS_OK;
@@ -413,6 +447,51 @@ int make_hilbert_table(Plan &p) {
   return SEIS_OK;
 }
 
+// Device memory of the arrays plan_create allocates (not the snapshots and
+// checkpoints, which come later).
+size_t plan_bytes(int op, int nshot, const seis_shot_desc *descs, int shape) {
+  const bool plane = op == OP_BORN_PLANE || op == OP_RTM_PLANE || op == OP_ILLUM_PLANE;
+  const bool born = op == OP_BORN || op == OP_BORN_PLANE, adj = op == OP_BORN_ADJ;
+  const bool rtm = op == OP_RTM || op == OP_RTM_TRUE || op == OP_RTM_UPDOWN;
+  size_t sum = 0, stage = 0, tiles = 0, cols = 0;
+  for (int s = 0; s < nshot; s++) {
+    const seis_shot_desc &d = descs[s];
+    const int NX = d.nx + 2 * d.pml, NZ = d.nz + 2 * d.pml, NT = d.nt + d.ndel;
+    const size_t f = Plan::rounded(sizeof(float) * field_geom(NX, NZ).elems);
+    const size_t model = (size_t)d.nx * d.nz, strip = LAYERS * 2 * ((size_t)d.nx + d.nz);
+    auto add = [&](size_t elems, size_t size) { sum += Plan::rounded(elems * size); };
+    // current fields, velocity; field B, perturbation; ring terms
+    sum += f * (3 + 1 + (born || rtm || op == OP_RTM_PLANE ? 3 : 0) + born + (adj ? 3 : 0));
+    if (plane) add((size_t)NT * d.nx, 4);
+    add(NT, 4);
+    add((size_t)d.nt * d.nx, 4);
+    add(d.nx, 4);
+    add(pad_tab_len(NX, NZ), 4);
+    if (rtm) add(d.nt * strip, 4);
+    if (op == OP_RTM_PLANE) add(NT * strip, 4);
+    if (op != OP_MODEL && !born) add(model, 4);
+    if (adj) {
+      add((size_t)d.nx * image_ld(d.nz, d.pml), 8);
+      add((size_t)EDGE_TAPS * edge_cells(NX, NZ), 4);
+      add(adj_tab_len(NX, NZ), 4);
+    }
+    if (op == OP_RTM_UPDOWN) {  // the four components; the Hilbert wavelet's table
+      add(4 * model, 4);
+      sum += 3 * f;
+      add(NT, 4);
+      add(d.nt * strip, 4);
+    }
+    stage = std::max(stage, std::max(model, (size_t)d.nx * (plane ? NT : d.nt)));
+    tiles += (size_t)((NX + shape_tx(shape) - 1) / shape_tx(shape)) *
+             ((NZ + shape_tz(shape) - 1) / shape_tz(shape));
+    cols += d.nx;
+  }
+  return sum + Plan::rounded(stage * 4) + 2 * Plan::rounded(tiles * sizeof(Tile)) +
+         2 * Plan::rounded((size_t)nshot * NMAPS * sizeof(CUtensorMap)) +
+         2 * Plan::rounded((size_t)nshot * sizeof(ShotDev)) + Plan::rounded(cols * sizeof(int2)) +
+         Plan::rounded(61 * 4);
+}
+
 int plan_create(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *descs, Plan **out,
                 int shape = SHAPE_32x64) {
   *out = nullptr;
@@ -440,7 +519,7 @@ int plan_create(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *descs
   p->nt = descs[0].nt;
   p->ndel = descs[0].ndel;
   p->NT = p->nt + p->ndel;
-  int rc = SEIS_OK;
+  int rc = p->reserve(plan_bytes(op, nshot, descs, shape));
   for (int s = 0; s < nshot && rc == SEIS_OK; s++) {
     const seis_shot_desc &d = descs[s];
     p->gz[s].assign(d.gz, d.gz + d.nx);
