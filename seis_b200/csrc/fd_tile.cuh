@@ -366,14 +366,36 @@ __device__ __forceinline__ bool in_range(float x) {
   const uint32_t lo = (uint32_t)(127 + LO) << 23, hi = (127u + 60u) << 23;
   return (__float_as_uint(x) & 0x7fffffffu) - lo <= hi - lo;
 }
+// n / d given rd = 1 / d rounded to nearest (1 <= d <= 2^30), for quotients
+// that the correction below cannot reach: a numerator below 2^-60 is divided
+// scaled by 2^90, where nothing underflows, and the quotient scaled back.
+// Below 2^-126 that rounds a second time; where the first rounding ended
+// half way between two results, the remainder's sign tells which side the
+// quotient lies on.
+__device__ __forceinline__ float quot_small(float n, float d, float rd, bool &ok) {
+  const bool t = fabsf(n) < 0x1p-60f;
+  const float N = n * (t ? 0x1p90f : 1.0f);
+  float q = N * rd;
+  ok = ok && (in_range<-100>(q) || n == 0.0f);
+  q = fmaf(fmaf(q, -d, N), rd, q);
+  q = fmaf(fmaf(q, -d, N), rd, q);
+  float o = q * (t ? 0x1p-90f : 1.0f);
+  const float e = fmaf(o, 0x1p90f, -q), rem = fmaf(q, -d, N);
+  if (t && fabsf(q) < 0x1p-36f && fabsf(e) == 0x1p-60f && rem != 0.0f)
+    o = (q + copysignf(0x1p-60f, rem)) * 0x1p-90f;
+  return n == 0.0f ? n : o;  // the sign of zero
+}
 // n / d of four rows given rd = 1 / d rounded to nearest: Markstein's
 // correction of an approximate quotient by its fused remainder (P. Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000
 // processor", 1990), which rounds correctly where nothing underflows or
-// overflows (1 <= d <= 2^30: from quotients of 2^-100 up); other quads (and
-// zero reciprocals, see ptab) divide.  Four quotients without a branch each:
-// the plain division tests every operand and takes its slow path for a zero
-// numerator, which is every pad cell that the wave has not reached.
+// overflows (1 <= d <= 2^30: from quotients of 2^-100 up), quads with smaller
+// quotients by quot_small; others (and zero reciprocals, see ptab) divide.
+// Four quotients without a branch each: the plain division tests every operand
+// and takes its slow path for a zero or tiny numerator, which is every pad
+// cell that the wave has not reached, and those just ahead of it: the pad
+// tiles that the front was crossing took 12,000 cycles for this phase instead
+// of 4,000, and a step waits for its slowest tile.
 __device__ __forceinline__ float4 quot_quad(const V4 &n, const V4 &d, const V4 &rd) {
   const V4 q0 = n * rd;
   const float4 q = f4(q0), N = f4(n);
@@ -388,7 +410,12 @@ __device__ __forceinline__ float4 quot_quad(const V4 &n, const V4 &d, const V4 &
     if (N.w == 0.0f) r.w = N.w;
     return r;
   }
-  return f4(n / d);
+  const float4 D = f4(d), R = f4(rd);
+  bool ok = true;
+  float4 r;
+#pragma unroll
+  for (int k = 0; k < 4; k++) set_comp(r, k, quot_small(comp(N, k), comp(D, k), comp(R, k), ok));
+  return ok ? r : f4(n / d);
 }
 #endif
 // 2 / x of four rows: the hardware's approximate reciprocal and two Newton

@@ -55,3 +55,25 @@ def test_pad_quads_match_restatement(ctx, nx, nz, pml, dt, amp, shape):
             got = p.get(0, OUT_GATHER)
         want = O.modeling(s, wav, vel) if op == OP_MODELING else O.born(s, wav, vel, dv)
         assert np.array_equal(got, want, equal_nan=True)
+
+
+@pytest.mark.parametrize("amp", [1e-33, 1e-36, 1e-39, 1e-42])
+def test_quotients_around_the_smallest_normal(ctx, amp):
+    """Pad cells whose one-way quotients cross the smallest normal number: the
+    scaled division and its second rounding, in the same bits."""
+    rng = np.random.default_rng(5)
+    s = Shot(nx=41, nz=37, pml=17, nt=90, ndel=4, sx=20, sz=3, dt=1e-3, dx=11.0, dz=9.0,
+             gz=rng.integers(0, 37, 41))
+    vel = (1500 + 2500 * rng.random((41, 37))).astype(np.float32)
+    dv = (40 * rng.standard_normal((41, 37))).astype(np.float32)
+    wav = (amp * rng.standard_normal(s.NT)).astype(np.float32)
+    for op in (OP_MODELING, OP_BORN):
+        with Plan(ctx, op, [s]) as p:
+            p.set(0, IN_VEL, vel)
+            p.set(0, IN_WAVELET, wav)
+            if op == OP_BORN:
+                p.set(0, IN_DV, dv)
+            p.run()
+            got = p.get(0, OUT_GATHER)
+        want = O.modeling(s, wav, vel) if op == OP_MODELING else O.born(s, wav, vel, dv)
+        assert np.array_equal(got, want)
