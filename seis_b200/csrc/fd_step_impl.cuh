@@ -157,7 +157,15 @@ cudaError_t launch_t(const ShotDev *d_shots, const Tile *d_tiles, int n_int, int
   constexpr int NT = Geo<S>::NT;
   const bool split = splits<S, MODE>(n_int, a.loop);
   if (split) {
-    const int G = LoopGrid<S, MODE>::ctas;
+    int G = LoopGrid<S, MODE>::ctas;
+    // Born's persistent CTAs (two of 112 KB per SM in the 256-thread shapes)
+    // leave no shared memory for a pad tile's CTA: beside pad tiles one per SM,
+    // which the memory-bound interior tiles hardly miss, so that the pad tiles,
+    // bound by latency and instructions, run beside them instead of after them
+    // (eight shots of 4000 x 1000: 151 -> 136 us a step, three: 54 -> 49).  The
+    // other modes' CTAs are smaller (one field: 1-2% either way; adjoint:
+    // slower), as are Born's in 32 x 32 tiles (slower).
+    if (MODE == MODE_BORN && LCfg<S, MODE>::MIN_CTAS == 2 && n_pad > 0 && s_int != s_pad) G /= 2;
     interior_loop_kernel<S, MODE><<<G < n_int ? G : n_int, NT, LCfg<S, MODE>::bytes, s_int>>>(
         d_shots, d_tiles, n_int, a, d_err);
     d_tiles += n_int;
