@@ -29,12 +29,6 @@
 namespace seis {
 namespace SEIS_NS {
 
-// 8th-order weight of offset m (|m| <= 4), fd.cpp:1245-1253
-__device__ __forceinline__ float tap8(int m) {
-  m = m < 0 ? -m : m;
-  return m == 0 ? SEIS_C4 : m == 1 ? SEIS_C3 : m == 2 ? SEIS_C2 : m == 3 ? SEIS_C1 : SEIS_C0;
-}
-
 // [t == s + 1] + [t == s - 1] - 2 [t == s]
 __device__ __forceinline__ float lap3(int t, int s) {
   return t == s ? -2.0f : (t == s + 1 || t == s - 1) ? 1.0f : 0.0f;

@@ -1410,11 +1410,11 @@ int64_t seis_fd_plan_launches_per_run(const seis_fd_plan *plan) {
 namespace {
 // 2 x `steps` time steps of the plan's step kernels (forward plans: the
 // operator's step; adjoint plans: the reverse step without imaging): first
-// the interior and the pad kernel one after the other, each bracketed by CUDA
-// events on its own stream, then `steps` steps as a run launches them (one
-// after the other, or concurrently on two streams when the plan overlaps
-// them).  ms = mean interior and pad kernel milliseconds (each
-// alone) and mean step milliseconds (as run); bytes = algorithmic bytes of
+// the interior and the pad tiles in a launch each, one after the other, each
+// bracketed by CUDA events on its own stream, then `steps` steps as a run
+// launches them (one launch of all tiles, or two, concurrently on two streams
+// when the plan overlaps them).  ms = mean milliseconds of the interior and of
+// the pad tiles (each alone) and mean step milliseconds (as run); bytes = algorithmic bytes of
 // the interior and pad tiles (16 per field cell-update).  The fields are
 // cleared afterwards.
 int time_steps(Plan &p, int steps, double *ms, double *bytes) {
@@ -1726,9 +1726,9 @@ static int run_batch(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *
   if (!in1 || !in2 || (what3 >= 0 && !in3) || !out)
     return fail(ctx, SEIS_ERR_ARG, "null array list");
   Plan *p = nullptr;
-  // one-field steps are fastest in 32x32 tiles (281 x 281: 8.7 us against 10.1 in
-  // 32x64; eight of 1280 x 480: 24.7 against 28.5), the adjoint's reverse step in 64x32
-  // (24.6 against 26.9 us), Born and RTM in 32x64 (15.0 against 15.7 us)
+  // one-field steps are fastest in 32x32 tiles (281 x 281: 6.6 us against 8.0 in
+  // 32x64; eight of 1280 x 480: 25.4 against 29.2), the adjoint's reverse step in 64x32
+  // (24.2 against 26.9 us), Born and RTM in 32x64 (11.5 against 11.7 us)
   const int shape = op == OP_MODEL || op == OP_ILLUM || op == OP_ILLUM_PLANE ? SHAPE_32x32
                     : op == OP_BORN_ADJ ? SHAPE_64x32 : SHAPE_32x64;
   rc = plan_create(ctx, op, nshot, shots, &p, shape);

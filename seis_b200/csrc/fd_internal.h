@@ -137,7 +137,8 @@ struct ShotDev {
 // ([7][NX rounded up]): top a2, a3, rd, bottom a2, a3, rd, weight; then per
 // corner (2 right + bottom) a3, its quotient's divisor d and rd.  a2 = hdt2 / v,
 // a3 = v / 4 / h / h, rd = 1 / (a1 + a2) or 1 / d, stored as zero outside
-// [2^-30, 1]; the contracted build keeps a1 + a2 in the place of rd.  Rows and columns beyond the grid repeat the last one.
+// [2^-30, 1]; the contracted build keeps a1 + a2 in the place of rd.  Rows and
+// columns beyond the grid repeat the last one.
 __host__ __device__ inline int pad_tab_nz(int NZ) { return (NZ + TZ_MAX - 1) / TZ_MAX * TZ_MAX; }
 __host__ __device__ inline int pad_tab_nx(int NX) { return (NX + TX_MAX - 1) / TX_MAX * TX_MAX; }
 __host__ __device__ inline int pad_tab_x(int NZ) { return 7 * pad_tab_nz(NZ); }  // by column
@@ -215,7 +216,7 @@ inline FieldGeom field_geom(int NX, int NZ) {
   return f;
 }
 
-// Kernel launchers (fd_kernels.cu, fd_step_*.cu, fd_adjoint_fast.cu).
+// Kernel launchers (fd_kernels.cu, fd_step_*.cu).
 enum StepMode : int {
   MODE_MODEL = 0,    // field A; point source; record; optional strip save
   MODE_RCV = 1,      // field B; receiver injection rec*vt2 (reference RTM)
@@ -223,10 +224,10 @@ enum StepMode : int {
   MODE_ADJ = 3,      // field A; reverse step of the exact Born adjoint (contracted build)
 };
 
-// One time step over every tile of a batch: the first n_int tiles are
-// interior tiles (one CTA each, stream s_int), the next n_pad pad tiles
-// (one CTA each, stream s_pad; the absorbing boundary fused in), tiles of
-// shape `shape` (TileShapeId).  `exact` selects the build that rounds like the
+// One time step over every tile of a batch: the first n_int tiles are interior
+// tiles, the next n_pad pad tiles (the absorbing boundary fused in), of shape
+// `shape` (TileShapeId); one launch on s_int, or the persistent interior kernel
+// there and the pad tiles on s_pad (step_splits).  `exact` selects the build that rounds like the
 // reference; otherwise the contracted build.
 cudaError_t launch_step(int mode, bool exact, const ShotDev *d_shots, const Tile *d_tiles,
                         int n_int, int n_pad, int shape, const StepArgs &a, int *d_err,
