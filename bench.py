@@ -319,15 +319,15 @@ def observed_data(ctx, sv):
 
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per cell of one
-# launch of each step kernel, from the ncu captures summarised in profiles/
-# (16 shots of the 1200 x 400 survey; Born kernels at 32 x 32 tiles, adjoint
-# kernels at 64 x 32); a launch's traffic is this times the cells it
-# updates (the captures' halo overhead is that of their tile shapes).
+# launch over the interior or the pad tiles, from the ncu capture summarised in
+# profiles/ (16 shots of the 1200 x 400 survey; Born at 32 x 64 tiles, adjoint
+# at 64 x 32); a launch's traffic is this times the cells it updates (the
+# capture's halo overhead is that of its tile shapes).
 NCU_TRAFFIC_PER_CELL = {
-    "born_interior": 215.0e6 / (6336 * 1024),
-    "born_pad": 141.0e6 / (3264 * 1024),
-    "adjoint_interior": 97.4e6 / (103809024 / 16),
-    "adjoint_pad": 127.2e6 / (1632 * 2048),
+    "born_interior": 193.3e6 / (2880 * 2048),
+    "born_pad": 168.6e6 / (2240 * 2048),
+    "adjoint_interior": 100.2e6 / (103809024 / 16),
+    "adjoint_pad": 130.9e6 / (1632 * 2048),
 }
 
 
@@ -335,8 +335,8 @@ def kernel_roofline(ctx, sv, iter_ms, launches_per_iter):
     """Per-kernel CUDA-event durations of the step kernels of one iteration --
     the Born step, the adjoint's reverse step and the source-field step it
     recomputes per checkpoint segment -- on separate plans over the same
-    shots: every kernel timed alone (interior tiles, then pad tiles), and the
-    step as a run launches it (both kernels, concurrently).  Returns the row
+    shots: the interior and the pad tiles each timed alone, and the step as a
+    run launches it.  Returns the row
     of the kernel with the largest share of the iteration (alone-time x
     launches), every row, and the autotuner's step times per tile shape."""
     from seis_b200._lib import (IN_DV, IN_VEL, IN_WAVELET, OP_BORN, OP_BORN_ADJOINT, OP_MODELING,
