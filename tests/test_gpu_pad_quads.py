@@ -8,7 +8,8 @@ import pytest
 
 import oracle as O
 from seis_b200 import Shot
-from seis_b200._lib import (IN_DV, IN_VEL, IN_WAVELET, LAUNCH_PER_TILE, OP_BORN, OP_MODELING,
+from seis_b200._lib import (IN_DV, IN_VEL, IN_WAVELET, LAUNCH_OVERLAP, LAUNCH_PER_TILE,
+                            LAUNCH_PERSISTENT, OP_BORN, OP_MODELING,
                             OUT_GATHER, TILE_SHAPES, Plan)
 
 pytestmark = pytest.mark.gpu
@@ -77,3 +78,25 @@ def test_quotients_around_the_smallest_normal(ctx, amp):
             got = p.get(0, OUT_GATHER)
         want = O.modeling(s, wav, vel) if op == OP_MODELING else O.born(s, wav, vel, dv)
         assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("shape", [k for k, v in sorted(TILE_SHAPES.items()) if v[0] * v[1] == 2048])
+def test_born_persistent_beside_pad_tiles(ctx, shape):
+    """Born's persistent interior kernel at one CTA per SM, with more interior
+    tiles than CTAs, beside the pad tiles: the restatement's bits."""
+    rng = np.random.default_rng(shape)
+    n = 800
+    s = Shot(nx=n, nz=n, pml=9, nt=10, ndel=2, sx=n // 2, sz=n // 2, dt=1e-3, dx=11.0, dz=9.0,
+             gz=n // 2 + rng.integers(-3, 4, n))
+    vel = (1500 + 2500 * rng.random((n, n))).astype(np.float32)
+    dv = (40 * rng.standard_normal((n, n))).astype(np.float32)
+    wav = rng.standard_normal(s.NT).astype(np.float32)
+    with Plan(ctx, OP_BORN, [s]) as p:
+        p.set_tile_shape(shape)
+        p.set_launch(LAUNCH_OVERLAP | LAUNCH_PERSISTENT)
+        p.set(0, IN_VEL, vel)
+        p.set(0, IN_WAVELET, wav)
+        p.set(0, IN_DV, dv)
+        p.run()
+        got = p.get(0, OUT_GATHER)
+    assert np.array_equal(got, O.born(s, wav, vel, dv))
