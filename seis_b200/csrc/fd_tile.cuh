@@ -240,10 +240,23 @@ __device__ __forceinline__ V4 operator-(const V4 &x) { return x * v4(-1.0f); }
 __device__ __forceinline__ V4 operator/(const V4 &x, const V4 &y) {
   return V4{make_float2(x.a.x / y.a.x, x.a.y / y.a.y), make_float2(x.b.x / y.b.x, x.b.y / y.b.y)};
 }
-// z + 2 x, z - 2 x: the doubling is exact, so the fused form rounds once as
-// the separate one does
-__device__ __forceinline__ V4 add_twice(const V4 &z, const V4 &x) { return fma4(x, v4(2.0f), z); }
-__device__ __forceinline__ V4 sub_twice(const V4 &z, const V4 &x) { return fma4(x, v4(-2.0f), z); }
+// z + 2 x, z - 2 x.  The doubling is exact, so the fused form rounds once as
+// the separate one does; only where 2 x overflows by itself do they part: the
+// exact build doubles first, as the reference does.
+__device__ __forceinline__ V4 add_twice(const V4 &z, const V4 &x) {
+#ifdef SEIS_FAST_MATH
+  return fma4(x, v4(2.0f), z);
+#else
+  return z + (x + x);
+#endif
+}
+__device__ __forceinline__ V4 sub_twice(const V4 &z, const V4 &x) {
+#ifdef SEIS_FAST_MATH
+  return fma4(x, v4(-2.0f), z);
+#else
+  return z - (x + x);
+#endif
+}
 // z + x y and z - x y as the build rounds them
 __device__ __forceinline__ V4 madd(const V4 &x, const V4 &y, const V4 &z) {
 #ifdef SEIS_FAST_MATH
