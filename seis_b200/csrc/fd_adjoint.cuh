@@ -135,12 +135,18 @@ __global__ void edge_coef_kernel(const ShotDev *__restrict__ shots, int nshots) 
 // cur, prev at the cell; _i at the inner neighbour, +-t along the strip), and
 // of a corner cell (fd.cpp:1146-1178) u31 = cz u3_z + cx u3_x + bK c.  atab
 // (ShotDev): per row of the left and right strip and per column of the top and
-// bottom strip al, be, ga; per corner cz, cx and bK.
+// bottom strip al, be, ga; per corner cz, cx and bK.  Without a pad there is no
+// strip cell and all are zero: the quads along the grid's edge take them times
+// a weight of zero, which a zero velocity's infinite ones would make NaN.
 __global__ void adj_tab_kernel(const ShotDev *__restrict__ shots) {
   const ShotDev &g = shots[blockIdx.y];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int NX = g.NX, NZ = g.NZ, n = adj_tab_nz(NZ), m = adj_tab_nx(NX);
   auto strip = [&](float *t, int stride, float v, float a1, float invh2) {
+    if (g.pml == 0) {
+      t[0] = t[stride] = t[2 * stride] = 0.0f;
+      return;
+    }
     const float rv = 1.0f / v, a2 = __fmul_rn(g.hdt2, rv), a3 = __fmul_rn(v * 0.25f, invh2);
     const float rd = 1.0f / __fadd_rn(a1, a2);
     t[0] = __fmul_rn(__fmaf_rn(-2.0f, a3, __fsub_rn(a1, a2)), rd);
@@ -163,9 +169,9 @@ __global__ void adj_tab_kernel(const ShotDev *__restrict__ shots) {
     const float ax3 = g.sqrt2f / v / g.dt;
     const float re = 1.0f / (g.ax1 + g.ax2 + ax3);
     float *t = g.atab + 6 * (n + m) + 4 * c;
-    t[0] = g.ax1 * re;
-    t[1] = g.ax2 * re;
-    t[2] = ax3 * re;
+    t[0] = g.pml == 0 ? 0.0f : g.ax1 * re;
+    t[1] = g.pml == 0 ? 0.0f : g.ax2 * re;
+    t[2] = g.pml == 0 ? 0.0f : ax3 * re;
     t[3] = 0.0f;
   }
 }
