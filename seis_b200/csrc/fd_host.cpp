@@ -70,12 +70,16 @@ int fail(seis_fd_ctx *ctx, int code, const char *fmt, ...) {
   return code;
 }
 
+// (a call's error stays the runtime's last error, which the next launch would
+// report as its own, until it is taken)
 #define CK(call)                                                                   \
   do {                                                                             \
     cudaError_t e_ = (call);                                                       \
-    if (e_ != cudaSuccess)                                                         \
+    if (e_ != cudaSuccess) {                                                       \
+      cudaGetLastError();                                                          \
       return fail(ctx, e_ == cudaErrorMemoryAllocation ? SEIS_ERR_NOMEM : SEIS_ERR_CUDA, \
                   "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+    }                                                                              \
   } while (0)
 
 int round_up(int x, int m) { return (x + m - 1) / m * m; }
