@@ -159,15 +159,21 @@ __device__ __forceinline__ float2 pair2(uint64_t r) {
 // of 320 rows: 210 -> 75 instructions a cell.
 // Then, when restore_it >= 0, the column's part of rtm_restore_kernel for the
 // next reverse step: nothing else reads these cells before it.
+// ZEROS = false: the column alone in shared memory, rows outside it by a test;
+// for columns that fit there without the zeros only (the last 66 rows up to
+// IMG_SMEM).
 constexpr int HILB_HALF = 30;
 constexpr int IMG_K = 3, IMG_THREADS = 128;
+constexpr size_t IMG_SMEM = 227 * 1024;  // the most a CTA can have
 // imaging of adjoint (lap vel3 R + FaQi), adjointPlane (FaQi of lap vel3),
 // rtm_true (FaQi of the source field times vel3)
 enum ImageMode { IMG_RTM = 0, IMG_PLANE = 1, IMG_TRUE = 2 };
+template <bool ZEROS>
 __global__ void __launch_bounds__(IMG_THREADS) rtm_image_kernel(
     const ShotDev *__restrict__ shots, const int2 *__restrict__ cols, int rot, int rot_b,
     const __grid_constant__ HilbertTaps taps, int mode, int restore_it) {
   extern __shared__ float2 sUR[];  // HILB_HALF zeros, the column, zeros
+  constexpr int H = ZEROS ? HILB_HALF : 0;  // the column's first row
   const int2 c = cols[blockIdx.x];
   const ShotDev &g = shots[c.x];
   const int ix = c.y + g.pml, NZ = g.NZ;
@@ -176,11 +182,13 @@ __global__ void __launch_bounds__(IMG_THREADS) rtm_image_kernel(
   const float *u2 = g.fa[rot % 3] + col, *r0 = g.fb[(rot_b + 2) % 3] + col;
   float *u1 = g.fa[(rot + 1) % 3] + col, *u0 = g.fa[(rot + 2) % 3] + col;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  for (int i = threadIdx.x; i < HILB_HALF; i += IMG_THREADS)
-    sUR[i] = make_float2(0.0f, 0.0f);
-  // up to a whole group of outputs past the last row
-  for (int i = HILB_HALF + NZ + threadIdx.x; i < NZ + 2 * HILB_HALF + 2 * IMG_K; i += IMG_THREADS)
-    sUR[i] = make_float2(0.0f, 0.0f);
+  if (ZEROS) {
+    for (int i = threadIdx.x; i < HILB_HALF; i += IMG_THREADS)
+      sUR[i] = make_float2(0.0f, 0.0f);
+    // up to a whole group of outputs past the last row
+    for (int i = H + NZ + threadIdx.x; i < NZ + 2 * HILB_HALF + 2 * IMG_K; i += IMG_THREADS)
+      sUR[i] = make_float2(0.0f, 0.0f);
+  }
   // before the wait what no step of the pass writes: vel3 into the field's
   // place, the layers to be restored towards L2.  With one shot the kernel is a
   // chain of memory latencies: with these loads and the image's taken off it, a
@@ -188,7 +196,7 @@ __global__ void __launch_bounds__(IMG_THREADS) rtm_image_kernel(
   // instead of 18.2.
   for (int iz = threadIdx.x; iz < NZ; iz += IMG_THREADS) {
     const float v = g.vel[col + iz];
-    sUR[HILB_HALF + iz].x = 2.0f / (v * v * v);
+    sUR[H + iz].x = 2.0f / (v * v * v);
   }
   const bool restore = restore_it >= 0 && restore_it < g.NT && restore_it >= g.ndel;
   const int edge = c.y < LAYERS ? c.y : c.y >= g.nx - LAYERS ? LAYERS + (g.nx - 1 - c.y) : -1;
@@ -206,7 +214,7 @@ __global__ void __launch_bounds__(IMG_THREADS) rtm_image_kernel(
 #pragma unroll
   for (int k = 0; k < IMG_K; k++) old[k] = zq + 2 * k < g.nz ? img0[zq + 2 * k] : 0.0f;
   for (int iz = threadIdx.x; iz < NZ; iz += IMG_THREADS) {
-    const float vel3 = sUR[HILB_HALF + iz].x;
+    const float vel3 = sUR[H + iz].x;
     float u;
     if (mode == IMG_TRUE) {  // rtm_true images the source field itself, fd.cpp:1014
       u = u0[iz] * vel3;
@@ -214,13 +222,13 @@ __global__ void __launch_bounds__(IMG_THREADS) rtm_image_kernel(
       const float lap = (u2[iz] + u0[iz] - 2.0f * u1[iz]) * g.idt2;
       u = lap * vel3;
     }
-    sUR[HILB_HALF + iz] = make_float2(u, r0[iz]);
+    sUR[H + iz] = make_float2(u, r0[iz]);
   }
   __syncthreads();
   const uint64_t nz = bits2(make_float2(IMG_NEG_ZERO, IMG_NEG_ZERO));
   for (int q = threadIdx.x; 2 * IMG_K * (q >> 1) + (q & 1) < g.nz; q += IMG_THREADS) {
     const int z0 = 2 * IMG_K * (q >> 1) + (q & 1);  // outputs z0, z0 + 2, ... (model rows)
-    const float2 *w = sUR + z0 + g.pml + 1;          // input z0 + pml - 29
+    const int in0 = z0 + g.pml - 29;                 // their first input
     uint64_t acc[IMG_K];
 #pragma unroll
     for (int k = 0; k < IMG_K; k++) acc[k] = 0;
@@ -228,7 +236,8 @@ __global__ void __launch_bounds__(IMG_THREADS) rtm_image_kernel(
     // tap h[30 - offset]; each output sums by increasing row
 #pragma unroll
     for (int m = 0; m < HILB_HALF + IMG_K - 1; m++) {
-      const uint64_t x = bits2(w[2 * m]);
+      const int row = in0 + 2 * m;
+      const uint64_t x = ZEROS || (row >= 0 && row < NZ) ? bits2(sUR[H + row]) : 0;
 #pragma unroll
       for (int k = 0; k < IMG_K; k++) {
         const int n = m - k;
@@ -241,7 +250,7 @@ __global__ void __launch_bounds__(IMG_THREADS) rtm_image_kernel(
     for (int k = 0; k < IMG_K; k++) {
       const int z = z0 + 2 * k;
       if (z >= g.nz) break;
-      const float2 ur = sUR[HILB_HALF + g.pml + z], f = pair2(acc[k]);
+      const float2 ur = sUR[H + g.pml + z], f = pair2(acc[k]);
       const float was = q == threadIdx.x ? old[k] : img0[z];
       float a = mode == IMG_RTM ? was + ur.x * ur.y : was;  // the others image with FaQi alone
       a = a + 0.5f * (ur.x * ur.y - f.x * f.y);
@@ -397,13 +406,14 @@ cudaError_t launch_rtm_restore(const ShotDev *d_shots, int nshots, int max_strip
   return cudaGetLastError();
 }
 
-cudaError_t launch_rtm_image(const ShotDev *d_shots, const int2 *d_cols, int ncols, int rot,
-                             int rot_b, int max_nz, const HilbertTaps &taps, cudaStream_t s,
-                             int mode, int restore_it, int pdl) {
-  const size_t smem = ((size_t)max_nz + 2 * HILB_HALF + 2 * IMG_K) * sizeof(float2);
+template <bool ZEROS>
+static cudaError_t launch_rtm_image_z(const ShotDev *d_shots, const int2 *d_cols, int ncols,
+                                      int rot, int rot_b, size_t smem, const HilbertTaps &taps,
+                                      cudaStream_t s, int mode, int restore_it, int pdl) {
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(rtm_image_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(rtm_image_kernel<ZEROS>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)std::max(smem, IMG_SMEM));
     if (e != cudaSuccess) return e;
   }
   cudaLaunchConfig_t c = {};
@@ -416,8 +426,19 @@ cudaError_t launch_rtm_image(const ShotDev *d_shots, const int2 *d_cols, int nco
   at[0].val.programmaticStreamSerializationAllowed = 1;
   c.attrs = at;
   c.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&c, rtm_image_kernel, d_shots, d_cols, rot, rot_b, taps, mode,
+  return cudaLaunchKernelEx(&c, rtm_image_kernel<ZEROS>, d_shots, d_cols, rot, rot_b, taps, mode,
                             restore_it);
+}
+cudaError_t launch_rtm_image(const ShotDev *d_shots, const int2 *d_cols, int ncols, int rot,
+                             int rot_b, int max_nz, const HilbertTaps &taps, cudaStream_t s,
+                             int mode, int restore_it, int pdl) {
+  const size_t column = (size_t)max_nz * sizeof(float2);
+  const size_t zeros = (2 * HILB_HALF + 2 * IMG_K) * sizeof(float2);
+  return column + zeros <= IMG_SMEM
+             ? launch_rtm_image_z<true>(d_shots, d_cols, ncols, rot, rot_b, column + zeros, taps, s,
+                                        mode, restore_it, pdl)
+             : launch_rtm_image_z<false>(d_shots, d_cols, ncols, rot, rot_b, column, taps, s, mode,
+                                         restore_it, pdl);
 }
 
 cudaError_t launch_updown_image(const ShotDev *d_shots, const ShotDev *d_shots_h,

@@ -1,5 +1,6 @@
-"""Reference RTM of columns longer than a CTA's shared memory holds: refused,
-and the next call is served."""
+"""Reference RTM of columns as long as a CTA's shared memory holds: with the
+filter's zeros around them (28,990 rows), without (up to 29,056), against the
+restatement, bit for bit; one row more is refused."""
 import numpy as np
 import pytest
 
@@ -20,6 +21,16 @@ def case(NZ):
     wav = rng.standard_normal(s.NT).astype(np.float32)
     rec = rng.standard_normal((nx, s.nt)).astype(np.float32)
     return s, wav, vel, rec
+
+
+@pytest.mark.parametrize("true", [False, True], ids=["adjoint", "rtm_true"])
+@pytest.mark.parametrize("NZ", [28990, 28991, 29024, 29056])
+def test_long_columns_match_restatement(ctx, NZ, true):
+    s, wav, vel, rec = case(NZ)
+    run, ref = (fd.rtm_true, O.rtm_true) if true else (fd.adjoint, O.rtm)
+    want = ref(s, wav, vel, rec)
+    assert np.abs(want).max() > 0
+    assert np.array_equal(run(*fd_args(s), wav, vel, rec, ctx=ctx), want)
 
 
 def test_longer_columns_are_refused(ctx):
