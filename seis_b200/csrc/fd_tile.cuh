@@ -1370,8 +1370,16 @@ __device__ __forceinline__ void tile_step(const ShotDev *__restrict__ shots, con
   pdl_wait();
   Imager im;
   if (K::ADJ) im.template load<TX, TZ>(g, a, t.x0, t.z0, ix, iz0);
+  // the copies of a CTA that gives up land before its shared memory is freed
+  // (waited for with a limit again)
+  auto give_up = [&]() {
+    if (tid != 0) return;
+    atomicExch(err, 1);
+    mbar_wait(bar, 0);
+    if (pad) mbar_wait(bar + 1, 0);
+  };
   if (!mbar_wait(bar, 0)) {
-    if (tid == 0) atomicExch(err, 1);
+    give_up();
     return;
   }
   if (pad) {
@@ -1380,7 +1388,7 @@ __device__ __forceinline__ void tile_step(const ShotDev *__restrict__ shots, con
       ok = adj_pad_cells<S>(g, a, t.x0, t.z0, sm, bar + 1, gzq, sort, corner, im);
     else
       ok = pad_cells<S, MODE>(g, a, t.x0, t.z0, sm, bar + 1, gzq, red);
-    if (!ok && tid == 0) atomicExch(err, 1);
+    if (!ok) give_up();
   } else {
     using SW = SAT<K::RW>;
     using ST = SAT<TZ>;
