@@ -1104,6 +1104,33 @@ int enqueue_operator(Plan &p) {
   return fail(p.ctx, SEIS_ERR_NOTSUP, "unknown operator %d", p.op);
 }
 
+// The launches of f() as a graph, and their number.
+template <class F>
+int capture(Plan &p, F f, cudaGraph_t *graph, int64_t *launches) {
+  seis_fd_ctx *ctx = p.ctx;
+  const int64_t before = ctx->launches;
+  CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+  int rc = f();
+  if (rc && p.overlap) {
+    // rejoin the auxiliary stream so that it leaves the capture with the
+    // main stream (an unjoined fork would keep it capturing)
+    cudaEventRecord(ctx->join, ctx->aux);
+    cudaStreamWaitEvent(ctx->stream, ctx->join, 0);
+  }
+  cudaGraph_t g = nullptr;
+  cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
+  *launches = ctx->launches - before;
+  ctx->launches = before;
+  if (rc || e != cudaSuccess) {
+    if (g) cudaGraphDestroy(g);
+    cudaGetLastError();
+    if (rc) return rc;
+  }
+  CK(e);
+  *graph = g;
+  return SEIS_OK;
+}
+
 int plan_run(Plan &p) {
   seis_fd_ctx *ctx = p.ctx;
   if (!p.exec) {
@@ -1120,27 +1147,9 @@ int plan_run(Plan &p) {
     if (rc0) return rc0;
   }
   if (!p.exec) {
-    int64_t before = ctx->launches;
-    CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = enqueue_operator(p);
-    if (rc && p.overlap) {
-      // rejoin the auxiliary stream so that it leaves the capture with the
-      // main stream (an unjoined fork would keep it capturing)
-      cudaEventRecord(ctx->join, ctx->aux);
-      cudaStreamWaitEvent(ctx->stream, ctx->join, 0);
-    }
-    cudaGraph_t g = nullptr;
-    cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
-    if (rc) {
-      if (g) cudaGraphDestroy(g);
-      cudaGetLastError();
-      return rc;
-    }
-    CK(e);
-    p.graph = g;
+    int rc = capture(p, [&] { return enqueue_operator(p); }, &p.graph, &p.launches_per_run);
+    if (rc) return rc;
     CK(cudaGraphInstantiate(&p.exec, p.graph, 0));
-    p.launches_per_run = ctx->launches - before;
-    ctx->launches = before;
   }
   CK(cudaGraphLaunch(p.exec, ctx->stream));
   ctx->launches += p.launches_per_run;
@@ -1413,97 +1422,126 @@ int64_t seis_fd_plan_launches_per_run(const seis_fd_plan *plan) {
 
 namespace {
 // 2 x `steps` time steps of the plan's step kernels (forward plans: the
-// operator's step; adjoint plans: the reverse step without imaging): first
-// the interior and the pad tiles in a launch each, one after the other, each
-// bracketed by CUDA events on its own stream, then `steps` steps as a run
-// launches them (one launch of all tiles, or two, concurrently on two streams
-// when the plan overlaps them).  ms = mean milliseconds of the interior and of
-// the pad tiles (each alone) and mean step milliseconds (as run); bytes = algorithmic bytes of
-// the interior and pad tiles (16 per field cell-update).  The fields are
-// cleared afterwards.
-int time_steps(Plan &p, int steps, double *ms, double *bytes) {
-  seis_fd_ctx *ctx = p.ctx;
-  const int TX = shape_tx(p.shape), TZ = shape_tz(p.shape);
-  const int mode = p.op == OP_BORN ? MODE_BORN : p.op == OP_BORN_ADJ ? MODE_ADJ : MODE_MODEL;
-  const bool exact = p.exact && mode != MODE_ADJ;
-  int fields = p.op == OP_BORN ? 2 : 1;
-  cudaEvent_t ev[5];
-  for (auto &e : ev) CK(cudaEventCreate(&e));
-  const bool adj = p.op == OP_BORN_ADJ;
-  const std::vector<Tile> &tl = adj ? p.adj_tiles : p.tiles;
-  const int n_int = adj ? p.n_int_adj : p.n_int, n_pad = adj ? p.n_pad_adj : p.n_pad;
-  const Tile *d_tl = adj ? p.d_adj_tiles : p.d_tiles;
-  int64_t cells_int = 0, cells_pad = 0;
-  for (size_t i = 0; i < tl.size(); i++) {
-    const Tile &t = tl[i];
-    const ShotDev &g = p.sd[t.shot];
-    int64_t c = (int64_t)std::min(TX, g.NX - t.x0) * std::min(TZ, g.NZ - t.z0);
-    ((int)i < n_int ? cells_int : cells_pad) += c;
+// operator's forward step; adjoint plans: the reverse step without imaging):
+// first the interior and the pad tiles in a launch each, one after the other,
+// each bracketed by CUDA events on its own stream, then `steps` steps as a run
+// launches them -- step() after step() in a graph, between one pair of events:
+// an event or a wait of the host between two steps would hold up the next
+// step's launch, which a run has in flight by then.  ms = mean milliseconds of
+// the interior and of the pad tiles (each alone, with the whole GPU: Born's
+// persistent kernel at two CTAs per SM, where a step beside pad tiles has one)
+// and mean step milliseconds (as run); bytes = algorithmic bytes of the
+// interior and pad tiles (16 per field cell-update).  The fields are cleared
+// afterwards.
+struct StepTimer {
+  cudaEvent_t ev[4] = {};
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  ~StepTimer() {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+    for (cudaEvent_t e : ev)
+      if (e) cudaEventDestroy(e);
   }
-  {
-    int rc0 = adj ? adj_tables(p) : pad_tabs(p);
-    if (rc0) return rc0;
-  }
+};
+// step k of the timed steps
+StepArgs timed_step(const Plan &p, int k) {
   StepArgs a{};
   a.nshots = p.nshot;
-  a.strip_k = -1;
   a.loop = p.loop;
   a.maps = p.d_maps;
-  // the interior tiles (the list's first n_int) or the pad tiles alone, on
-  // the main / auxiliary stream
-  auto launch = [&](bool interior) -> cudaError_t {
-    const int ni = interior ? n_int : 0, np = interior ? 0 : n_pad;
-    const Tile *t0 = interior ? d_tl : d_tl + n_int;
-    return launch_step(mode, exact, p.d_sd, t0, ni, np, p.shape, a, ctx->d_err, ctx->stream,
-                       ctx->aux);
+  a.rot = k;
+  a.rot_b = k;
+  const int it = k % p.NT;
+  a.src_k = it >= 1 ? it - 1 : -1;
+  a.rec_k = it - p.ndel >= 0 && p.op != OP_RTM && p.op != OP_BORN_ADJ ? it - p.ndel : -1;
+  return a;
+}
+int step_mode(const Plan &p) {
+  return p.op == OP_BORN ? MODE_BORN : p.op == OP_BORN_ADJ ? MODE_ADJ : MODE_MODEL;
+}
+// mean milliseconds of steps k0 .. k0 + steps - 1 as a run launches them
+int time_as_run(Plan &p, int k0, int steps, double *ms) {
+  seis_fd_ctx *ctx = p.ctx;
+  StepTimer t;
+  for (int i = 0; i < 2; i++) CK(cudaEventCreate(&t.ev[i]));
+  int64_t n = 0;
+  auto chain = [&]() -> int {
+    CK(cudaEventRecordWithFlags(t.ev[0], ctx->stream, cudaEventRecordExternal));
+    for (int k = k0; k < k0 + steps; k++) {
+      StepArgs a = timed_step(p, k);
+      a.pdl = k > k0;
+      int rc = step(p, step_mode(p), a);
+      if (rc) return rc;
+    }
+    CK(cudaEventRecordWithFlags(t.ev[1], ctx->stream, cudaEventRecordExternal));
+    return SEIS_OK;
   };
-  double t_int = 0, t_pad = 0, t_step = 0;
-  for (int k = 0; k < 2 * steps; k++) {
-    const bool alone = k < steps;  // first each kernel alone, then the step as it runs
-    a.rot = k; a.rot_b = k;
-    int it = k % p.NT;
-    a.src_k = it >= 1 ? it - 1 : -1;
-    a.rec_k = it - p.ndel >= 0 && p.op != OP_RTM && !adj ? it - p.ndel : -1;
-    CK(cudaEventRecord(ev[0], ctx->stream));
-    if (alone) {
-      CK(launch(true));
-      CK(cudaEventRecord(ev[1], ctx->stream));
-      CK(cudaEventRecord(ev[2], ctx->stream));
-      CK(cudaStreamWaitEvent(ctx->aux, ev[2], 0));
-      CK(launch(false));
-      CK(cudaEventRecord(ev[3], ctx->aux));
-      CK(cudaStreamWaitEvent(ctx->stream, ev[3], 0));
-    } else if (p.overlap) {
-      CK(cudaStreamWaitEvent(ctx->aux, ev[0], 0));
-      CK(launch_step(mode, exact, p.d_sd, d_tl, n_int, n_pad, p.shape, a, ctx->d_err, ctx->stream,
-                     ctx->aux));
-      CK(cudaEventRecord(ev[3], ctx->aux));
-      CK(cudaStreamWaitEvent(ctx->stream, ev[3], 0));
-    } else {
-      CK(launch_step(mode, exact, p.d_sd, d_tl, n_int, n_pad, p.shape, a, ctx->d_err, ctx->stream,
-                     ctx->stream));
-    }
-    CK(cudaEventRecord(ev[4], ctx->stream));
-    CK(cudaEventSynchronize(ev[4]));
-    if (alone) {
-      float a1 = 0, a2 = 0;
-      CK(cudaEventElapsedTime(&a1, ev[0], ev[1]));
-      CK(cudaEventElapsedTime(&a2, ev[2], ev[3]));
-      t_int += a1; t_pad += a2;
-    } else {
-      float a3 = 0;
-      CK(cudaEventElapsedTime(&a3, ev[0], ev[4]));
-      t_step += a3;
-    }
-    ctx->launches += 2;
+  int rc = capture(p, chain, &t.graph, &n);
+  if (rc) return rc;
+  CK(cudaGraphInstantiate(&t.exec, t.graph, 0));
+  CK(cudaGraphUpload(t.exec, ctx->stream));
+  CK(cudaGraphLaunch(t.exec, ctx->stream));
+  ctx->launches += n;
+  CK(cudaStreamSynchronize(ctx->stream));
+  float sum = 0;
+  CK(cudaEventElapsedTime(&sum, t.ev[0], t.ev[1]));
+  *ms = sum / steps;
+  return SEIS_OK;
+}
+// mean milliseconds of the interior and of the pad tiles of the same steps,
+// each alone
+int time_alone(Plan &p, int steps, double *ms) {
+  seis_fd_ctx *ctx = p.ctx;
+  const bool adj = p.op == OP_BORN_ADJ, exact = p.exact && !adj;
+  const int n_int = adj ? p.n_int_adj : p.n_int, n_pad = adj ? p.n_pad_adj : p.n_pad;
+  const Tile *d_tl = adj ? p.d_adj_tiles : p.d_tiles;
+  StepTimer t;
+  for (cudaEvent_t &e : t.ev) CK(cudaEventCreate(&e));
+  for (int k = 0; k < steps; k++) {
+    const StepArgs a = timed_step(p, k);
+    CK(cudaEventRecord(t.ev[0], ctx->stream));
+    CK(launch_step(step_mode(p), exact, p.d_sd, d_tl, n_int, 0, p.shape, a, ctx->d_err,
+                   ctx->stream, ctx->aux));
+    CK(cudaEventRecord(t.ev[1], ctx->stream));
+    CK(cudaEventRecord(t.ev[2], ctx->stream));
+    CK(cudaStreamWaitEvent(ctx->aux, t.ev[2], 0));
+    CK(launch_step(step_mode(p), exact, p.d_sd, d_tl + n_int, 0, n_pad, p.shape, a, ctx->d_err,
+                   ctx->stream, ctx->aux));
+    CK(cudaEventRecord(t.ev[3], ctx->aux));
+    CK(cudaStreamWaitEvent(ctx->stream, t.ev[3], 0));
+    CK(cudaEventSynchronize(t.ev[3]));
+    float a1 = 0, a2 = 0;
+    CK(cudaEventElapsedTime(&a1, t.ev[0], t.ev[1]));
+    CK(cudaEventElapsedTime(&a2, t.ev[2], t.ev[3]));
+    ms[0] += a1 / steps;
+    ms[1] += a2 / steps;
+    ctx->launches += (n_int > 0) + (n_pad > 0);
   }
-  for (auto &e : ev) cudaEventDestroy(e);
-  ms[0] = t_int / steps; ms[1] = t_pad / steps; ms[2] = t_step / steps;
+  return SEIS_OK;
+}
+int time_steps(Plan &p, int steps, double *ms, double *bytes) {
+  const int TX = shape_tx(p.shape), TZ = shape_tz(p.shape);
+  const int fields = p.op == OP_BORN ? 2 : 1;
+  const bool adj = p.op == OP_BORN_ADJ;
+  ms[0] = ms[1] = ms[2] = 0.0;
+  int rc = adj ? adj_tables(p) : pad_tabs(p);
+  if (!rc) rc = time_alone(p, steps, ms);
+  if (!rc) rc = time_as_run(p, steps, steps, &ms[2]);
+  if (rc) return rc;
   if (bytes) {
-    bytes[0] = 16.0 * fields * (double)cells_int;
-    bytes[1] = 16.0 * fields * (double)cells_pad;
+    const std::vector<Tile> &tl = adj ? p.adj_tiles : p.tiles;
+    const int n_int = adj ? p.n_int_adj : p.n_int;
+    bytes[0] = bytes[1] = 0.0;
+    for (size_t i = 0; i < tl.size(); i++) {
+      const Tile &t = tl[i];
+      const ShotDev &g = p.sd[t.shot];
+      const int64_t c = (int64_t)std::min(TX, g.NX - t.x0) * std::min(TZ, g.NZ - t.z0);
+      bytes[(int)i < n_int ? 0 : 1] += 16.0 * fields * (double)c;
+    }
   }
-  return clear_fields(p) ? SEIS_ERR_CUDA : sync(ctx);
+  rc = clear_fields(p);
+  return rc ? rc : sync(p.ctx);
 }
 
 // Switch a plan to tile shape s: tile lists, tensor-map boxes and
