@@ -289,14 +289,16 @@ int seis_fd_plan_set_launch(seis_fd_plan *plan, int flags);
 int seis_fd_plan_launch(const seis_fd_plan *plan);
 /* Autotuner: time `steps` steps of the plan's own kernels (as
  * seis_fd_plan_time_kernels, on its current inputs) in every tile shape and
- * launch form (one tile per CTA or persistent, one after the other or
- * overlapped), and keep the fastest.  The choice is cached in the
- * process per plan signature (operator, build flavour, every shot's padded
- * grid) and reused by later plans of the same signature unless `force` is
- * set.  Adjoint plans with FP16 snapshots stay at 64x32 (the snapshots' scales
- * belong to the tiles).  h_ms[SEIS_TILE_SHAPES] (may be null) receives each shape's shortest
- * mean step time (0 where not timed), *h_best (may be null) the shape kept.
- * The plan's fields are clobbered. */
+ * every launch form that differs there (one launch of all tiles; persistent,
+ * one after the other or overlapped, where a shape leaves interior tiles), and
+ * keep the fastest.  Plans of the reference's RTM are timed by their forward
+ * step.  The choice is cached in the process per plan signature (operator,
+ * build flavour, every shot's padded grid) and reused by later plans of the
+ * same signature unless `force` is set.  Adjoint plans with FP16 snapshots stay
+ * at 64x32 (the snapshots' scales belong to the tiles); their other shapes are
+ * timed only when h_ms is given.  h_ms[SEIS_TILE_SHAPES] (may be null) receives
+ * each shape's shortest mean step time (0 where not timed), *h_best (may be
+ * null) the shape kept.  The plan's fields are clobbered. */
 int seis_fd_plan_autotune(seis_fd_plan *plan, int steps, int force, double *h_ms, int *h_best);
 
 /* Batched forms of the single-shot calls: h_*[i] are the arrays of shot i. */

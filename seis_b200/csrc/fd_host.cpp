@@ -1615,11 +1615,11 @@ void set_launch(Plan &p, bool overlap, int loop) {
   p.graph = nullptr;
 }
 
-// Time `steps` steps of the plan in every tile shape and launch form (the
-// interior kernel one tile per CTA or persistent, the interior and pad
-// kernels one after the other or concurrently) and keep the fastest (the
-// cached choice for this plan's signature unless `force`).  ms: the shortest
-// mean step time of every shape (0 where not timed), may be null.
+// Time `steps` steps of the plan in every tile shape and launch form (one
+// launch of all tiles, or the persistent interior kernel with the pad tiles
+// after or beside it) and keep the fastest (the cached choice for this plan's
+// signature unless `force`).  ms: the shortest mean step time of every shape (0
+// where not timed), may be null.
 int autotune(Plan &p, int steps, bool force, double *ms, int *best) {
   const std::string key = tune_key(p);
   if (ms)
@@ -1642,28 +1642,31 @@ int autotune(Plan &p, int steps, bool force, double *ms, int *best) {
   // choice by time would change its results in their last bits from one
   // process to the next.  Such a plan stays at 64x32, the fastest shape of
   // most surveys from a hundred to some thousand tiles and within 10% of the
-  // fastest in the others; its launch form is chosen by time.
+  // fastest in the others; its launch form is chosen by time.  Its other shapes
+  // are timed for a caller that asks for their times only.
   const bool steady = fp16_scales(p);
-  int pick = 0, pick_steady = 0;
-  double t_best = 0.0, t_steady = 0.0;
+  int pick = -1;
+  double t_best = 0.0;
   for (int c = 0; c < 4 * NSHAPES; c++) {
+    const int s = c >> 2;
+    const bool eligible = !steady || s == SHAPE_64x32;
+    if (!eligible && !ms) continue;
     int rc = apply(c);
+    if (rc) return rc;
+    // without the persistent kernel, or without interior tiles for it, a step
+    // is the same one launch in every form: timed once, as a new plan's (1)
+    const int n_int = p.op == OP_BORN_ADJ ? p.n_int_adj : p.n_int;
+    if ((c & 3) != 1 && (!(c & 2) || n_int == 0)) continue;
     double t[3];
-    if (!rc) rc = time_steps(p, 3, t, nullptr);  // warm-up
+    rc = time_steps(p, 3, t, nullptr);  // warm-up
     if (!rc) rc = time_steps(p, steps, t, nullptr);
     if (rc) return rc;
-    const int s = c >> 2;
     if (ms && (ms[s] == 0.0 || t[2] < ms[s])) ms[s] = t[2];
-    if (c == 0 || t[2] < t_best) {
+    if (eligible && (pick < 0 || t[2] < t_best)) {
       t_best = t[2];
       pick = c;
     }
-    if (s == SHAPE_64x32 && (t_steady == 0.0 || t[2] < t_steady)) {
-      t_steady = t[2];
-      pick_steady = c;
-    }
   }
-  if (steady) pick = pick_steady;
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     g_tune_cache[key] = pick;
