@@ -295,8 +295,9 @@ int seis_fd_plan_launch(const seis_fd_plan *plan);
  * step.  The choice is cached in the process per plan signature (operator,
  * build flavour, every shot's padded grid) and reused by later plans of the
  * same signature unless `force` is set.  Adjoint plans with FP16 snapshots stay
- * at 64x32 (the snapshots' scales belong to the tiles); their other shapes are
- * timed only when h_ms is given.  h_ms[SEIS_TILE_SHAPES] (may be null) receives
+ * at 64x32 (the snapshots' scales belong to the tiles), also when they are set
+ * to FP16 after this call; their other shapes are timed only when h_ms is
+ * given.  h_ms[SEIS_TILE_SHAPES] (may be null) receives
  * each shape's shortest mean step time (0 where not timed), *h_best (may be
  * null) the shape kept.  The plan's fields are clobbered. */
 int seis_fd_plan_autotune(seis_fd_plan *plan, int steps, int force, double *h_ms, int *h_best);

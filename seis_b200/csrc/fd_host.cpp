@@ -152,6 +152,7 @@ struct Plan {
   // (else one after the other on the main stream)
   bool overlap = true;
   int loop = -1;  // interior kernel form (StepArgs::loop)
+  bool by_time = false;  // the tile shape is the autotuner's choice by time
   std::vector<void *> allocs;
   std::vector<size_t> alloc_bytes;
   // one cleared allocation that alloc() carves the plan's arrays from (what
@@ -1626,6 +1627,7 @@ int autotune(Plan &p, int steps, bool force, double *ms, int *best) {
     for (int s = 0; s < NSHAPES; s++) ms[s] = 0.0;
   // choice = 4 shape + 2 persistent + overlap
   auto apply = [&](int c) {
+    p.by_time = !fp16_scales(p);
     set_launch(p, (c & 1) != 0, (c >> 1) & 1);
     return apply_shape(p, c >> 2);
   };
@@ -1685,7 +1687,9 @@ int seis_fd_plan_time_kernels(seis_fd_plan *plan, int steps, double *ms, double 
 int seis_fd_plan_set_tile_shape(seis_fd_plan *plan, int shape) {
   if (!plan || !plan->p) return SEIS_ERR_ARG;
   int rc = begin(plan->p->ctx);
-  return rc ? rc : apply_shape(*plan->p, shape);
+  if (!rc) rc = apply_shape(*plan->p, shape);
+  if (!rc) plan->p->by_time = false;
+  return rc;
 }
 
 int seis_fd_plan_tile_shape(const seis_fd_plan *plan) {
@@ -1727,7 +1731,12 @@ int seis_fd_plan_set_snapshots(seis_fd_plan *plan, int every, int dtype) {
                 every, p.ck_every);
   p.snap_every = every;
   p.snap_dtype = dtype;
-  return SEIS_OK;
+  if (!fp16_scales(p) || !p.by_time) return SEIS_OK;
+  // a shape chosen by time for other snapshots gives way to FP16's (autotune)
+  int rc = begin(p.ctx);
+  if (!rc) rc = apply_shape(p, SHAPE_64x32);
+  if (!rc) p.by_time = false;
+  return rc;
 }
 
 int seis_fd_plan_set_checkpoints(seis_fd_plan *plan, int every) {

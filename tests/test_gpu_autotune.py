@@ -7,7 +7,7 @@ import pytest
 
 import oracle as O
 from seis_b200 import Shot
-from seis_b200._lib import (IN_VEL, IN_WAVELET, OP_BORN_ADJOINT, OP_MODELING, SNAP_F16, TILE_64x32,
+from seis_b200._lib import (IN_VEL, IN_WAVELET, OP_BORN_ADJOINT, OP_MODELING, SNAP_F16, TILE_16x128, TILE_64x32,
                             TILE_SHAPES, Plan)
 
 pytestmark = pytest.mark.gpu
@@ -48,3 +48,18 @@ def test_fp16_adjoint_times_its_own_shape(ctx):
         n, best = launches(ctx, p, ms)  # times asked for
         assert n == len(TILE_SHAPES) * ONE[OP_BORN_ADJOINT] and all(t > 0 for t in ms)
         assert best == p.tile_shape == TILE_64x32
+
+
+def test_fp16_after_tuning_takes_its_shape(ctx):
+    """FP16 set after a tuning by time: the plan's shape is FP16's all the same
+    (sizes of which not every one is fastest in 64x32); a shape set by hand stays."""
+    for n in (21, 60, 130, 300):
+        with plan(ctx, OP_BORN_ADJOINT, n) as p:
+            p.autotune(steps=STEPS, force=True)
+            p.set_snapshots(2, SNAP_F16)
+            assert p.tile_shape == TILE_64x32
+    with plan(ctx, OP_BORN_ADJOINT) as p:
+        p.autotune(steps=STEPS, force=True)
+        p.set_tile_shape(TILE_16x128)
+        p.set_snapshots(2, SNAP_F16)
+        assert p.tile_shape == TILE_16x128
