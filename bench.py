@@ -320,14 +320,14 @@ def observed_data(ctx, sv):
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per cell of one
 # launch over the interior or the pad tiles, from the ncu capture summarised in
-# profiles/ (16 shots of the 1200 x 400 survey; Born at 32 x 64 tiles, adjoint
-# at 64 x 32); a launch's traffic is this times the cells it updates (the
-# capture's halo overhead is that of its tile shapes).
+# profiles/ (16 shots of the 1200 x 400 survey), with the capture's tile shape;
+# a launch's traffic is this times the cells it updates, and not given for
+# another shape (the halo's share is the shape's).
 NCU_TRAFFIC_PER_CELL = {
-    "born_interior": 193.3e6 / (2880 * 2048),
-    "born_pad": 168.6e6 / (2240 * 2048),
-    "adjoint_interior": 100.2e6 / (103809024 / 16),
-    "adjoint_pad": 130.9e6 / (1632 * 2048),
+    "born_interior": ("32x64", 193.3e6 / (2880 * 2048)),
+    "born_pad": ("32x64", 168.6e6 / (2240 * 2048)),
+    "adjoint_interior": ("64x32", 100.2e6 / (103809024 / 16)),
+    "adjoint_pad": ("64x32", 130.9e6 / (1632 * 2048)),
 }
 
 
@@ -335,43 +335,59 @@ def kernel_roofline(ctx, sv, iter_ms, launches_per_iter):
     """Per-kernel CUDA-event durations of the step kernels of one iteration --
     the Born step, the adjoint's reverse step and the source-field step it
     recomputes per checkpoint segment -- on separate plans over the same
-    shots: the interior and the pad tiles each timed alone, and the step as a
-    run launches it.  Returns the row
-    of the kernel with the largest share of the iteration (alone-time x
-    launches), every row, and the autotuner's step times per tile shape."""
+    shots, in the solver's tile shapes and launch forms: the interior and the
+    pad tiles each timed alone (with the whole GPU), and the step as a run
+    launches it.  Returns the row of the kernel with the largest share of the
+    iteration (alone-time x launches), every row, and the autotuner's step times
+    per tile shape."""
     from seis_b200._lib import (IN_DV, IN_VEL, IN_WAVELET, OP_BORN, OP_BORN_ADJOINT, OP_MODELING,
-                                TILE_SHAPES, Plan)
+                                SNAP_F16, TILE_SHAPES, Plan)
     wav = sv.wavelet()
-    rows, tuning = [], {}
+    rows, tuning, adjoint = [], {}, None
     for op, name in ((OP_BORN, "born"), (OP_BORN_ADJOINT, "adjoint"), (OP_MODELING, "source")):
         n = launches_per_iter.get(name, 0)
         if not n:
             continue
         with Plan(ctx, op, sv.shots) as p:
-            if op != OP_BORN_ADJOINT:
-                p.set_exact(False)  # the solver's forward operators run the fast build
+            # as the solver's plans: the build and the snapshots' type are part of
+            # the tuning's signature
+            p.set_exact(False)
+            if op == OP_BORN_ADJOINT:
+                p.set_snapshots(SNAP_EVERY, SNAP_F16)
             for i in range(len(sv.shots)):
                 p.set(i, IN_VEL, sv.sub(sv.vel0, i))
                 p.set(i, IN_WAVELET, wav)
                 if op == OP_BORN:
                     p.set(i, IN_DV, sv.sub(sv.dv, i))
             if op != OP_MODELING:
-                # the autotuner's step time of every tile shape on these shots
-                # (the solver's plans of the same signature use the same choice)
-                best, per_shape = p.autotune(steps=10, force=True)
-                tuning[name] = {"chosen": "%dx%d" % TILE_SHAPES[best],
+                # the choice made for the solver's plan of the same signature,
+                # then the step times of every tile shape on these shots
+                p.autotune(steps=10)
+                kept = p.tile_shape, p.launch
+                _, per_shape = p.autotune(steps=10, force=True)
+                p.set_tile_shape(kept[0])
+                p.set_launch(kept[1])
+                tuning[name] = {"chosen": "%dx%d" % TILE_SHAPES[kept[0]],
                                 "step_ms": {"%dx%d" % TILE_SHAPES[k]: v
                                             for k, v in enumerate(per_shape)}}
+                if op == OP_BORN_ADJOINT:
+                    adjoint = kept
+            elif adjoint:  # recomputed by the adjoint's plan
+                p.set_tile_shape(adjoint[0])
+                p.set_launch(adjoint[1])
+            shape = "%dx%d" % TILE_SHAPES[p.tile_shape]
             p.time_kernels(10)
             ms, by = p.time_kernels(100)
         per_cell = 32.0 if op == OP_BORN else 16.0
         for k, kname in ((0, "interior"), (1, "pad")):
             kern = f"{name}_{kname}"
-            tr = NCU_TRAFFIC_PER_CELL.get(kern)
-            rows.append({"kernel": kern, "ms": ms[k], "bytes": by[k], "launches_per_iter": n,
-                         "share": ms[k] * n / iter_ms, "GB_s": by[k] / (ms[k] * 1e6),
-                         "traffic": tr * by[k] / per_cell if tr else None, "timed": "alone"})
-        rows.append({"kernel": f"{name}_step", "ms": ms[2], "bytes": by[0] + by[1],
+            at, tr = NCU_TRAFFIC_PER_CELL.get(kern, (None, None))
+            rows.append({"kernel": kern, "shape": shape, "ms": ms[k], "bytes": by[k],
+                         "launches_per_iter": n, "share": ms[k] * n / iter_ms,
+                         "GB_s": by[k] / (ms[k] * 1e6),
+                         "traffic": tr * by[k] / per_cell if at == shape else None,
+                         "timed": "alone"})
+        rows.append({"kernel": f"{name}_step", "shape": shape, "ms": ms[2], "bytes": by[0] + by[1],
                      "launches_per_iter": n, "share": ms[2] * n / iter_ms,
                      "GB_s": (by[0] + by[1]) / (ms[2] * 1e6), "timed": "as run"})
     kern = [r for r in rows if not r["kernel"].endswith("_step")]
