@@ -534,9 +534,9 @@ __device__ __forceinline__ bool adj_pad_cells(const ShotDev &g, const StepArgs &
       const int bza = b == 1 ? max(za, NZ - 5) : za, bzb = b == 0 ? min(zb, 5) : zb;
       const int nr = bzb - bza, nc = bxb - bxa;
       if (nr <= 0 || nc <= 0) continue;
-      const float rn = 1.0f / (float)nr;  // see CellList
+      const float rn = 1.0f / (float)nr;  // see quot
       for (int i = tid; i < nr * nc; i += NT_T) {
-        const int q = CellList::quot(i, rn);
+        const int q = quot(i, rn);
         const int cx = bxa + q, cz = bza + (i - q * nr);
         const float *c = g.edge_coef + edge_index(b, NX, NZ, cx, cz);
         float s = 0.0f;

@@ -467,9 +467,6 @@ __device__ __forceinline__ float4 scatter_source(const float4 &vel, const float4
   return f4(t * t * v4(lap) * two_over(v * v * v) * v4(dv));
 }
 __device__ __forceinline__ float4 add4(const float4 &x, const float4 &y) { return f4(v4(x) + v4(y)); }
-__device__ __forceinline__ float4 ldg4(const float *p) {
-  return __ldg(reinterpret_cast<const float4 *>(p));
-}
 
 // Write this thread's source-term values (lap of the background field) of
 // snapshot `k`: two column quads (columns ix, ix + 1 from row iz0), the rows of
@@ -543,60 +540,10 @@ struct GA {
   }
 };
 
-// The grid cells of a tile [x0, x0 + TX) x [z0, z0 + TZ) that lie outside a
-// rectangle [rx0, rx1) x [rz0, rz1) (the model, or the model less its edge
-// cells), enumerated column by column, z fastest, so that the threads of a
-// CTA can share them evenly and consecutive threads touch consecutive rows.
-// Column indices come from a float reciprocal: for i < 2^13 and column
-// lengths of at most 128, (i + 0.5) / len lies at least 0.5 / len = 2^-8 from
-// an integer and the rounded product within 2^-10 of it, so its floor is the
-// integer quotient.
-struct CellList {
-  int x0, z0, xe, ze;  // tile cells inside the grid: [x0, xe) x [z0, ze)
-  int ma, mb;          // tile columns crossing the rectangle: [ma, mb)
-  int top, bot;        // cells of such a column above / below the rectangle
-  int cp, cm, n;       // cells per other column, per crossing column, in all
-  float rcp, rcm;      // 1 / cp, 1 / cm
-  __device__ __forceinline__ CellList(int x0_, int z0_, int xe_, int ze_, int rx0, int rx1,
-                                      int rz0, int rz1)
-      : x0(x0_), z0(z0_), xe(xe_), ze(ze_) {
-    ma = min(max(rx0, x0), xe);
-    mb = min(max(rx1, ma), xe);
-    top = max(0, min(ze, rz0) - z0);
-    bot = max(0, ze - max(z0, rz1));
-    if (rz1 <= rz0) top = ze - z0, bot = 0;  // empty rectangle: whole columns
-    cp = ze - z0;
-    cm = top + bot;
-    n = (xe - x0 - (mb - ma)) * cp + (mb - ma) * cm;
-    rcp = cp > 0 ? 1.0f / (float)cp : 0.0f;
-    rcm = cm > 0 ? 1.0f / (float)cm : 0.0f;
-  }
-  static __device__ __forceinline__ int quot(int i, float r) {
-    return (int)(((float)i + 0.5f) * r);
-  }
-  __device__ __forceinline__ void cell(int i, int &cx, int &cz) const {
-    const int na = (ma - x0) * cp;
-    if (i < na) {
-      const int q = quot(i, rcp);
-      cx = x0 + q;
-      cz = z0 + (i - q * cp);
-      return;
-    }
-    i -= na;
-    const int nm = (mb - ma) * cm;
-    if (i < nm) {
-      const int q = quot(i, rcm);
-      cx = ma + q;
-      const int r = i - q * cm;
-      cz = r < top ? z0 + r : ze - bot + (r - top);
-      return;
-    }
-    i -= nm;
-    const int q = quot(i, rcp);
-    cx = mb + q;
-    cz = z0 + (i - q * cp);
-  }
-};
+// i / len given r = 1 / len as the build divides (within two units in the last
+// place), for i < 2^13: (i + 0.5) / len lies at least 0.5 / len from an integer,
+// the rounded product within 2^13 / len * 2^-21 = 2^-8 / len of it.
+__device__ __forceinline__ int quot(int i, float r) { return (int)(((float)i + 0.5f) * r); }
 
 // Two-way values of a pad tile and its one-cell halo in shared memory:
 // columns x0-1 .. x0+TX, rows z0-4 .. z0+TZ+3 (U3R = TZ + 8 rows per column;
@@ -630,8 +577,8 @@ __device__ __forceinline__ void halo_cell(int i, int x0, int z0, int &hx, int &h
 
 // Row quads [4q, 4q + 3] of a tile's columns that hold at least one grid cell
 // outside a rectangle [rx0, rx1) x [rz0, rz1) (the model, or the model less its
-// edge cells), enumerated column by column, rows fastest (see
-// CellList).
+// edge cells), enumerated column by column, rows fastest, so that the threads
+// of a CTA can share them evenly (indices by quot).
 struct QuadList {
   int x0, xe;      // tile columns inside the grid
   int ma, mb;      // tile columns crossing the model: [ma, mb)
@@ -660,7 +607,7 @@ struct QuadList {
       i -= na;
       const int nm = (mb - ma) * cm;
       if (i < nm) {
-        q = CellList::quot(i, rcm);
+        q = quot(i, rcm);
         cx = ma + q;
         const int r = i - q * cm;
         dz = 4 * (r < top ? r : cp - bot + (r - top));
@@ -669,7 +616,7 @@ struct QuadList {
       i -= nm;
       base = mb;
     }
-    q = CellList::quot(i, rcp);
+    q = quot(i, rcp);
     cx = base + q;
     dz = 4 * (i - q * cp);
   }
