@@ -320,13 +320,14 @@ def observed_data(ctx, sv):
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per cell of one
 # launch over the interior or the pad tiles, from the ncu capture summarised in
-# profiles/ (16 shots of the 1200 x 400 survey), with the capture's tile shape;
-# a launch's traffic is this times the cells it updates, and not given for
-# another shape (the halo's share is the shape's).
+# profiles/ (16 shots of the 1200 x 400 survey; interior tiles by the persistent
+# kernel, as the large survey runs them), with the capture's tile shape; a
+# launch's traffic is this times the cells it updates, and not given for another
+# shape (the halo's share is the shape's).
 NCU_TRAFFIC_PER_CELL = {
-    "born_interior": ("32x64", 193.3e6 / (2880 * 2048)),
+    "born_interior": ("32x64", 189.0e6 / (2880 * 2048)),
     "born_pad": ("32x64", 168.6e6 / (2240 * 2048)),
-    "adjoint_interior": ("64x32", 100.2e6 / (103809024 / 16)),
+    "adjoint_interior": ("64x32", 97.6e6 / (103809024 / 16)),
     "adjoint_pad": ("64x32", 130.9e6 / (1632 * 2048)),
 }
 

@@ -53,7 +53,11 @@ typedef struct seis_fd_plan seis_fd_plan;
  * minus the arrays. */
 typedef struct {
   int nx, nz;     /* model (aperture) extent, cells */
-  int pml;        /* absorbing pad width, cells (>= 1) */
+  int pml;        /* absorbing pad width, cells (>= 1; 0 runs without a pad, with
+                   * one difference: what is added to the grid's edge cells,
+                   * Born's scattering source and RTM's receivers in the first
+                   * and last column, counts, where the reference overwrites
+                   * it) */
   int nt;         /* recorded samples */
   int ndel;       /* steps simulated before recording starts */
   int sx, sz;     /* source cell, unpadded indices */
@@ -280,7 +284,9 @@ int seis_fd_plan_tile_shape(const seis_fd_plan *plan);
  * persistent form when each of its CTAs gets at least 4 tiles.
  * SEIS_LAUNCH_OVERLAP: the two launches of the persistent form concurrently on
  * two streams (else one after the other on the context's stream).
- * A new plan has SEIS_LAUNCH_OVERLAP. */
+ * The reverse steps of SEIS_OP_RTM and SEIS_OP_RTM_TRUE have one form whatever
+ * the flags, all tiles of both fields in one launch; the flags hold for their
+ * forward steps.  A new plan has SEIS_LAUNCH_OVERLAP. */
 #define SEIS_LAUNCH_OVERLAP 1
 #define SEIS_LAUNCH_PERSISTENT 2
 #define SEIS_LAUNCH_PER_TILE 4

@@ -634,8 +634,6 @@ int plan_create(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *descs
   return SEIS_OK;
 }
 
-// Upload an unpadded [nx][nz] model of shot s into a padded device field.
-
 // The absorbing coefficients of every shot's pad strips, from the velocities as
 // they are now; before the first step of a run.
 int pad_tabs(Plan &p) {
@@ -820,8 +818,11 @@ int run_rtm_reverse(Plan &p) {
   StepArgs a{};
   a.nshots = p.nshot;
   a.maps = p.d_maps;
-  // the imaging kernel also prepares the next step, where the boundary layers
-  // of a model do not meet
+  // Both fields' tiles go in one launch in every form: a whole run of eight
+  // 1200 x 400 shots takes 32.7 ms with it beside one-launch forward steps, 33.2
+  // beside persistent ones; with the two fields in turn, persistent, it took 46.
+  // The imaging kernel also prepares the next step, where the boundary layers
+  // of a model do not meet.
   bool chain = true;
   for (const ShotDev &g : p.sd) chain = chain && std::min(g.nx, g.nz) >= 2 * LAYERS;
   int k = 0;
@@ -1642,10 +1643,11 @@ int autotune(Plan &p, int steps, bool force, double *ms, int *best) {
   // An adjoint plan's shape is also the tiling of its FP16 snapshots' scales,
   // and small values lie in FP16's denormal range by their tile's scale: a
   // choice by time would change its results in their last bits from one
-  // process to the next.  Such a plan stays at 64x32, the fastest shape of
-  // most surveys from a hundred to some thousand tiles and within 10% of the
-  // fastest in the others; its launch form is chosen by time.  Its other shapes
-  // are timed for a caller that asks for their times only.
+  // process to the next.  Such a plan stays at 64x32: a reverse step there takes
+  // 12.2 us of one 817x320 shot (32x64: 12.6), 21.8 of four 1280x480 (21.7), 46
+  // of eight (41) and 121 of four 4080x1080 (107).  Its launch form is chosen by
+  // time.  Its other shapes are timed for a caller that asks for
+  // their times only.
   const bool steady = fp16_scales(p);
   int pick = -1;
   double t_best = 0.0;
@@ -1780,9 +1782,10 @@ static int run_batch(seis_fd_ctx *ctx, int op, int nshot, const seis_shot_desc *
   if (!in1 || !in2 || (what3 >= 0 && !in3) || !out)
     return fail(ctx, SEIS_ERR_ARG, "null array list");
   Plan *p = nullptr;
-  // one-field steps are fastest in 32x32 tiles (281 x 281: 6.6 us against 8.0 in
-  // 32x64; eight of 1280 x 480: 25.4 against 29.2), the adjoint's reverse step in 64x32
-  // (24.2 against 26.9 us), Born and RTM in 32x64 (11.5 against 11.7 us)
+  // one-field steps are fastest in 32x32 tiles (281 x 281: 8.0 us against 8.7 in
+  // 32x64; eight of 1280 x 480: 25.5 against 29.3), one shot's adjoint in 64x32
+  // (817 x 320: 12.2 against 12.6), Born and RTM in 32x64 (11.6 against 11.8 in
+  // 32x32; 16 RTM shots 123 against 128 us per step of the whole pass)
   const int shape = op == OP_MODEL || op == OP_ILLUM || op == OP_ILLUM_PLANE ? SHAPE_32x32
                     : op == OP_BORN_ADJ ? SHAPE_64x32 : SHAPE_32x64;
   rc = plan_create(ctx, op, nshot, shots, &p, shape);
@@ -2024,8 +2027,6 @@ int lsrtm_shape(seis_fd_lsrtm &L, Plan &p) {
   return autotune(p, 10, false, nullptr, nullptr);
 }
 
-// s = L^T r: adjoint plan over the residuals, per-shot images scattered into
-// the global grid.
 // The plan of shots k0 .. k1-1 of a grouped solver: velocity sub-grids and
 // wavelet from the device copies; an adjoint plan reads the residual.
 int lsrtm_group_plan(seis_fd_lsrtm &L, int op, int k0, int k1, Plan **out) {

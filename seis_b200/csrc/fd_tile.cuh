@@ -1219,8 +1219,8 @@ __device__ __forceinline__ bool pad_cells(const ShotDev &g, const StepArgs &a, i
 // copies of what no step changes (velocity, perturbation, coefficient table)
 // are issued before the wait for the last step, those of the fields after it.
 // Measured per step (before: interior and pad kernels on two streams): one
-// 281 x 281 shot 18.6 -> 6.6 us, Born 817 x 320 27 -> 11.5 us, eight 1280 x 480
-// shots in the exact build 57 -> 25 us (16 B per cell at the copy rate: 12 us);
+// 281 x 281 shot 18.6 -> 6.7 us, Born 817 x 320 27 -> 11.6 us, eight 1280 x 480
+// shots in the exact build 57 -> 25.5 us (16 B per cell at the copy rate: 12 us);
 // the pad tiles of eight Born shots of 4000 x 1000: 84 -> 68 us.
 template <int S, int MODE>
 __device__ __forceinline__ void tile_step(const ShotDev *__restrict__ shots, const Tile &t,
