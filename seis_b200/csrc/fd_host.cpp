@@ -1462,15 +1462,15 @@ StepArgs timed_step(const Plan &p, int k) {
 int step_mode(const Plan &p) {
   return p.op == OP_BORN ? MODE_BORN : p.op == OP_BORN_ADJ ? MODE_ADJ : MODE_MODEL;
 }
-// mean milliseconds of steps k0 .. k0 + steps - 1 as a run launches them
-int time_as_run(Plan &p, int k0, int steps, double *ms) {
+// milliseconds of steps k0 .. k1 - 1 as a run launches them
+int time_chain(Plan &p, int k0, int k1, float *ms) {
   seis_fd_ctx *ctx = p.ctx;
   StepTimer t;
   for (int i = 0; i < 2; i++) CK(cudaEventCreate(&t.ev[i]));
   int64_t n = 0;
   auto chain = [&]() -> int {
     CK(cudaEventRecordWithFlags(t.ev[0], ctx->stream, cudaEventRecordExternal));
-    for (int k = k0; k < k0 + steps; k++) {
+    for (int k = k0; k < k1; k++) {
       StepArgs a = timed_step(p, k);
       a.pdl = k > k0;
       int rc = step(p, step_mode(p), a);
@@ -1486,8 +1486,19 @@ int time_as_run(Plan &p, int k0, int steps, double *ms) {
   CK(cudaGraphLaunch(t.exec, ctx->stream));
   ctx->launches += n;
   CK(cudaStreamSynchronize(ctx->stream));
-  float sum = 0;
-  CK(cudaEventElapsedTime(&sum, t.ev[0], t.ev[1]));
+  CK(cudaEventElapsedTime(ms, t.ev[0], t.ev[1]));
+  return SEIS_OK;
+}
+// mean milliseconds of `steps` steps from k0 on, in graphs of a bounded size
+int time_as_run(Plan &p, int k0, int steps, double *ms) {
+  constexpr int CHUNK = 4096;
+  double sum = 0.0;
+  for (int k = 0; k < steps; k += CHUNK) {
+    float part = 0.0f;
+    int rc = time_chain(p, k0 + k, k0 + std::min(steps, k + CHUNK), &part);
+    if (rc) return rc;
+    sum += part;
+  }
   *ms = sum / steps;
   return SEIS_OK;
 }
